@@ -72,7 +72,8 @@ bool listed(const int (&list)[N], int v) {
 // Overrides of a new plan's algorithms for measurement and testing, read
 // from CURADON_GB300_ALGO: comma-separated key=value tokens, e.g.
 // "fwd2d=tex,bwd2d_minb=48".  Keys: fwd2d = alu | tex | cslab |
-// cslab<443 | 474 | 484>; bwd2d = alu | tex | smem; bwd2d_minb = 27 | 48 | 68
+// cslab<443 | 474 | 484>; fwd2d_bundle = small | large (the chunked forward's
+// bundles); bwd2d = alu | tex | smem; bwd2d_minb = 27 | 48 | 68
 // (staged backprojector variants); adj2d = pair | quad; fwd3d = alu | tex3 |
 // quad | mixed; fwd3d_tex = 0..8 (texture warps of 8 in the mixed forward);
 // fwd3d_unroll = 1 | 2 (samples per iteration of the quad / mixed forward);
@@ -109,6 +110,10 @@ void apply_algo_env(Plan2d *p2, Plan3d *p3) {
                 for (int k : kFwdChunkShapes)
                     if (val == "cslab" + std::to_string(k)) p2->fwd_chunk_rows = k;
             }
+        }
+        if (p2 && key == "fwd2d_bundle") {
+            if (val == "small") p2->fwd_bundle = -1;
+            if (val == "large") p2->fwd_bundle = 1;
         }
         if (p2 && key == "bwd2d") {
             if (val == "alu") p2->algo_bwd = 0;
@@ -308,6 +313,16 @@ bool finite_all(const float *a, uint64_t n) {
     for (uint64_t i = 0; i < n; ++i)
         if (!std::isfinite(a[i])) return false;
     return true;
+}
+
+// Median absolute difference of consecutive directions, modulo a full turn.
+template <class Dir>
+double median_step(uint64_t n, Dir dir) {
+    if (n < 2) return 0.0;
+    std::vector<double> d(n - 1);
+    for (uint64_t i = 0; i + 1 < n; ++i) d[i] = std::fabs(std::remainder(dir(i + 1) - dir(i), 2 * M_PI));
+    std::nth_element(d.begin(), d.begin() + (n - 1) / 2, d.end());
+    return d[(n - 1) / 2];
 }
 
 int check_device(int device) {
@@ -582,6 +597,7 @@ int cg_plan2d_create(cg_plan2d **plan, int device, uint32_t vol_prec, const uint
     // less time than the texture unit at 704^2, 11 % at 768^2, 25 % at
     // 1024^2, 39 % at 2048^2; even at 640^2, 5 % more at 512^2
     if ((long long)p->W * p->H >= 704LL * 704) p->algo_fwd = 4;
+    p->view_step = median_step(nangles, [&](uint64_t i) { return (double)angles[i]; });
     apply_algo_env(p.get(), nullptr);
     int rc = CG_OK;
     auto fail = [&](int code) {
@@ -641,6 +657,9 @@ int cg_plan2d_create_vec(cg_plan2d **plan, int device, uint32_t vol_prec,
     p->device = device;
     p->vec = true;
     if ((long long)p->W * p->H >= 704LL * 704) p->algo_fwd = 4;
+    p->view_step = median_step(nangles, [&](uint64_t i) {
+        return std::atan2((double)vecs[6 * i + 5], (double)vecs[6 * i + 4]);
+    });
     apply_algo_env(p.get(), nullptr);
     p->algo_bwd = 2;  // the staged backprojector is the one driven by the projective table
     int rc = CG_OK;

@@ -115,6 +115,11 @@ struct Plan2d {
     // 474 (the same staged by per-lane cp.async) or 443 ((v, d) pairs, pair
     // reuse, view groups four views apart); the autotuner's candidates
     int fwd_chunk_rows = 484;
+    // median angle between consecutive views (radians), for the chunked
+    // forward's choice of bundle; fwd_bundle -1 / 1 forces the small / large
+    // one (CURADON_GB300_ALGO fwd2d_bundle=small / large)
+    double view_step = 0;
+    int fwd_bundle = 0;
     // staged backprojector's variant: 68 (default: packed FP32 row pairs,
     // floor by FP32 adds, window rows by bulk copies, absolute-position
     // pairs, 8 x 4-pixel warps), 48 (the same staged pair by pair with
@@ -333,10 +338,8 @@ int launch_backward2d_smem(const Plan2d &p, float *vol, cudaStream_t s);
 // blocks of the quarter-turn backprojection of a W x W image
 int sym_quadrant_blocks(int W);
 int sm_count();
-// rows: the chunked forward's compiled shape (kFwdChunkShapes: 443, 474,
-// 484); views [v0, v0 + nv), all by default
-int launch_forward2d_cslab(const Plan2d &p, float *sino, cudaStream_t s, int rows, int v0 = 0,
-                           int nv = -1);
+// rows: the chunked forward's compiled shape (kFwdChunkShapes: 443, 474, 484)
+int launch_forward2d_cslab(const Plan2d &p, float *sino, cudaStream_t s, int rows);
 // The plan's 2D volume texture array and object (allocated once).
 int ensure_vol_texture(Plan2d &p);
 // the first `active` problems of a batch (the work list's blocks [0, total))

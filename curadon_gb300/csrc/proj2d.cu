@@ -16,6 +16,7 @@
 #include <algorithm>
 #include <cfloat>
 #include <climits>
+#include <cmath>
 
 #include "common.cuh"
 
@@ -611,17 +612,31 @@ __device__ __forceinline__ void cslab_bundle(const float2 *__restrict__ layA,
                 }
             }
         } else {
+            // a window wider than the buffer: the samples from global memory,
+            // GR rows of a ray at a time with their loads issued together (one
+            // row at a time, each waited for, was the longest part of a
+            // sparse-view bundle: 1024^2 x 360 views 470 -> 426 us; four rays
+            // per thread have registers for two rows, 2048^2 x 2048: 4501 us
+            // at one, 4435 at two, 4541 at eight)
+            constexpr int GR = GV > 2 ? 2 : 8;
             const unsigned gcap = (unsigned)(pmaxi + kPad);
 #pragma unroll
             for (int g = 0; g < GV; ++g) {
-                const int ra = max(r0, rlo[g]), rb = min(r0 + K - 1, rlo[g] + len[g] - 1);
-                for (int r = ra; r <= rb; ++r) {
-                    float fp;
-                    const unsigned c = cs_column<ABS>(p[g], -kPad - ic, gcap, fp);
-                    const float2 *rowp = lay + (size_t)(r + kPad) * pitch;
-                    const float2 lo = __ldg(rowp + c), hi = __ldg(rowp + pitch + c);
-                    acc[g].add(fp, lo, hi);
-                    p[g] += V[g];
+                const int ra = max(r0, rlo[g]), rb = min(r0 + K, rlo[g] + len[g]);
+                for (int rg = ra; rg < rb; rg += GR) {
+                    float fp[GR];
+                    float2 lo[GR], hi[GR];
+#pragma unroll
+                    for (int k = 0; k < GR; ++k) {
+                        // rows past the ray's last are loaded from it and dropped
+                        const unsigned c = cs_column<ABS>(p[g], -kPad - ic, gcap, fp[k]);
+                        const float2 *rowp = lay + (size_t)(min(rg + k, rb - 1) + kPad) * pitch + c;
+                        lo[k] = __ldg(rowp), hi[k] = __ldg(rowp + pitch);
+                        if (rg + k < rb) p[g] += V[g];
+                    }
+#pragma unroll
+                    for (int k = 0; k < GR; ++k)
+                        if (rg + k < rb) acc[g].add(fp[k], lo[k], hi[k]);
                 }
             }
         }
@@ -667,23 +682,45 @@ __global__ void __launch_bounds__(T * VS, MB)
 
 }  // namespace
 
-int launch_forward2d_cslab(const Plan2d &p, float *sino, cudaStream_t s, int rows, int v0,
-                           int nv) {
-    // views [v0, v0 + nv): the kernel sees offset tables and sinogram rows
-    if (nv < 0) nv = p.nangles - v0;
-    if (nv <= 0) return CG_OK;
-    const int ng = 8;  // views per bundle of the compiled shapes
-    const int groups = ceil_div(nv, ng);
-    if (groups > 65535) return set_error(CG_ERR_INVALID, "too many views for one launch");
+// Rows per chunk and pair columns of the two bundles' windows (two buffers
+// each): 8 views x 128 cells (three blocks of 256 threads per SM) and 4 views
+// x 64 cells (five blocks of 128).
+constexpr int kCsRows = 16, kCsCols = 256, kCsSmallCols = 144;
+static size_t cslab_smem(int stride) { return 2 * sizeof(float2) * (kCsRows + 1) * stride; }
+
+// Which bundle the chunked forward takes (the sums are the same bits).  The
+// large one shares each window among twice the views and cells, which pays
+// while neighbouring views overlap and there are bundles for every SM.  Its
+// end views lie 7 view steps apart, i.e. up to 7 step R pixels at the image's
+// corners (R half its diagonal): past about 90 the windows outgrow their
+// buffer and read global memory.  Below three rounds of resident blocks the
+// last round is mostly idle and the small bundles' finer blocks fill it.
+// Large / small in us: sparse views 2048^2 x 360 (177 px) 1497 / 1222, 768^2
+// x 200 (120 px) 257 / 154; 2048^2 x 900 (71 px) 2294 / 2456; few bundles
+// 1024^2 x 360 (1.2 rounds) 428 / 352, 900^2 x 900 (2.5) 591 / 574; dense
+// 1024^2 x 1024 (3.4 rounds, 31 px) 749 / 790, 2048^2 x 2048 4435 / 5287.
+// Batches keep the large one for all: a second launch for some problems'
+// small bundles has a last round of its own (twelve problems of 192^2 ..
+// 1024^2 with their gradient: 2495 us with it).
+static bool cslab_small(const Plan2d &p) {
+    if (p.fwd_bundle) return p.fwd_bundle < 0;
+    const double spread = 7.0 * p.view_step * 0.5 * std::hypot((double)p.W, (double)p.H);
+    const long long bundles = (long long)ceil_div(p.det, 128) * ceil_div(p.nangles, 8);
+    return spread > 90.0 || bundles < 3LL * 3 * sm_count();
+}
+
+int launch_forward2d_cslab(const Plan2d &p, float *sino, cudaStream_t s, int rows) {
+    if (ceil_div(p.nangles, 8) > 65535)
+        return set_error(CG_ERR_INVALID, "too many views for one launch");
     if (std::max(p.pitchA(), p.pitchB()) >= 32768)
         return set_error(CG_ERR_INVALID, "volume too wide for the chunked forward");
-    auto go = [&](auto kernel, int k, int stride, int cells, int vs = 1) -> int {
-        const size_t smem = 2 * sizeof(float2) * (k + 1) * stride;
+    auto go = [&](auto kernel, int stride, int cells, int views) -> int {
+        const size_t smem = cslab_smem(stride);
         if (int rc = ensure_smem_attr((const void *)kernel, (int)smem)) return rc;
-        dim3 grid(ceil_div(p.det, cells), groups, 2);
-        kernel<<<grid, cells * vs, smem, s>>>(p.d_layA, p.d_layB, sino + (size_t)v0 * p.det,
-                                           p.d_src + v0, p.d_u0 + v0, p.d_du + v0, p.W, p.H,
-                                           p.det, nv, p.sx, p.sy, p.pitchA(), p.pitchB());
+        dim3 grid(ceil_div(p.det, cells), ceil_div(p.nangles, views), 2);
+        kernel<<<grid, cells * 2, smem, s>>>(p.d_layA, p.d_layB, sino, p.d_src, p.d_u0, p.d_du,
+                                             p.W, p.H, p.det, p.nangles, p.sx, p.sy, p.pitchA(),
+                                             p.pitchB());
         CG_TRY_CUDA(cudaGetLastError());
         return CG_OK;
     };
@@ -691,9 +728,14 @@ int launch_forward2d_cslab(const Plan2d &p, float *sino, cudaStream_t s, int row
     // staged by per-lane cp.async, 6 % slower at n=2048; 443: (v, d) pairs,
     // pair reuse, view groups four views apart, 30 % slower)
     switch (rows) {
-        case 443: return go(k_fwd2d_cslab<16, 256, 128, true, true, 2, 8, 3, 1>, 16, 256, 128, 2);
-        case 474: return go(k_fwd2d_cslab<16, 256, 128, true, false, 2, 8, 3, 2, true>, 16, 256, 128, 2);
-        case 484: return go(k_fwd2d_cslab<16, 256, 128, true, false, 2, 8, 3, 2, true, true>, 16, 256, 128, 2);
+        case 443: return go(k_fwd2d_cslab<16, 256, 128, true, true, 2, 8, 3, 1>, kCsCols, 128, 8);
+        case 474: return go(k_fwd2d_cslab<16, 256, 128, true, false, 2, 8, 3, 2, true>, kCsCols, 128, 8);
+        case 484:
+            if (cslab_small(p) && ceil_div(p.nangles, 4) <= 65535)
+                return go(k_fwd2d_cslab<kCsRows, kCsSmallCols, 64, true, false, 2, 4, 5, 2, true, true>,
+                          kCsSmallCols, 64, 4);
+            return go(k_fwd2d_cslab<kCsRows, kCsCols, 128, true, false, 2, 8, 3, 2, true, true>,
+                      kCsCols, 128, 8);
         default: return set_error(CG_ERR_INVALID, "unknown chunk shape");
     }
 }
@@ -1338,7 +1380,7 @@ __global__ void __launch_bounds__(256, 3)
     const Prob2d &q = probs[i];
     const int local = blockIdx.x - start[i];
     const int gx = (q.det + 127) / 128, gy = (q.nangles + 7) / 8;
-    cslab_bundle<16, 256, 128, true, false, 2, 8, 3, 2, true, true>(
+    cslab_bundle<kCsRows, kCsCols, 128, true, false, 2, 8, 3, 2, true, true>(
         q.layA, q.layB, q.sino, q.src, q.u0, q.du, q.W, q.H, q.det, q.nangles, q.sx, q.sy, q.pa,
         q.pb, local % gx, (local / gx) % gy, local / (gx * gy));
 }
@@ -1430,8 +1472,8 @@ int launch_batch2d_fwd_plans(const Prob2d *d_probs, const std::vector<Prob2d> &p
     k_batch_relayout2d_abs<<<totals[7], dim3(32, 8), 0, s>>>(d_probs, starts + 7 * (count + 1),
                                                              count);
     CG_TRY_CUDA(cudaGetLastError());
-    constexpr int smem = 2 * (int)sizeof(float2) * (16 + 1) * 256;
-    if ((rc = ensure_smem_attr((const void *)k_batch_fwd2d_cslab, smem))) return rc;
+    const size_t smem = cslab_smem(kCsCols);
+    if ((rc = ensure_smem_attr((const void *)k_batch_fwd2d_cslab, (int)smem))) return rc;
     k_batch_fwd2d_cslab<<<totals[8], 256, smem, s>>>(d_probs, starts + 8 * (count + 1), count);
     CG_TRY_CUDA(cudaGetLastError());
     return CG_OK;
