@@ -21,7 +21,9 @@
 // same work list.  Each problem uses its own
 // plan's scratch, so a plan may appear in one batch only once, and a batch
 // must not overlap on the GPU with other calls on its plans.
+#include <algorithm>
 #include <memory>
+#include <numeric>
 #include <set>
 #include <string>
 #include <vector>
@@ -38,6 +40,14 @@ struct cg_batch2d {
     int *d_starts = nullptr;  // kBatchStages stages x (count + 1)
     int totals[cg::kBatchStages] = {};
     std::vector<int> starts;  // host copy of d_starts
+    // the same work list with the problems of the longest blocks first, for
+    // launches over all problems: forward (blocks as long as the rays) and
+    // backprojection (as long as the views).  In the caller's order a long
+    // problem near the end leaves most SMs idle while its last blocks run
+    // (twelve problems of 192^2 .. 1024^2, 193 .. 715 views, us: forward 1557
+    // -> 1532, backprojection 814 -> 740; sixteen: 1730 -> 1708, 904 -> 811).
+    cg::Prob2d *d_sorted[2] = {};
+    int *d_sorted_starts[2] = {};
     int active = 0;           // problems [0, active) run (cg_batch2d_set_active)
     bool adjoint_ready = false;  // the plans' quad accumulators are bound
 
@@ -75,6 +85,32 @@ namespace {
 void free_batch(cg_batch2d *b) {
     if (b->d_probs) cudaFree(b->d_probs);
     if (b->d_starts) cudaFree(b->d_starts);
+    for (int k = 0; k < 2; ++k) {
+        if (b->d_sorted[k]) cudaFree(b->d_sorted[k]);
+        if (b->d_sorted_starts[k]) cudaFree(b->d_sorted_starts[k]);
+    }
+}
+
+// The work list of a batch in the given order of its problems, on the device.
+cudaError_t upload_work(const cg_batch2d &b, const std::vector<int> &order, Prob2d **d_probs,
+                        int **d_starts) {
+    const int n1 = b.count + 1;
+    std::vector<Prob2d> probs(b.count);
+    std::vector<int> starts(kBatchStages * n1, 0);
+    for (int k = 0; k < b.count; ++k) {
+        const int i = order[k];
+        probs[k] = b.probs[i];
+        for (int st = 0; st < kBatchStages; ++st)
+            starts[st * n1 + k + 1] =
+                starts[st * n1 + k] + b.starts[st * n1 + i + 1] - b.starts[st * n1 + i];
+    }
+    cudaError_t e;
+    if ((e = cudaMalloc(d_probs, sizeof(Prob2d) * b.count)) != cudaSuccess) return e;
+    if ((e = cudaMalloc(d_starts, sizeof(int) * starts.size())) != cudaSuccess) return e;
+    e = cudaMemcpy(*d_probs, probs.data(), sizeof(Prob2d) * b.count, cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) return e;
+    return cudaMemcpy(*d_starts, starts.data(), sizeof(int) * starts.size(),
+                      cudaMemcpyHostToDevice);
 }
 
 // floats of a problem's axial view tables (10 per view), rounded up so that
@@ -151,15 +187,19 @@ int cg_batch2d_create(cg_batch2d **batch, cg_plan2d *const *plans, float *const 
         return set_error(e == cudaErrorMemoryAllocation ? CG_ERR_NOMEM : CG_ERR_CUDA,
                          std::string("batch set-up: ") + cudaGetErrorString(e));
     };
+    std::vector<int> order(count);
+    std::iota(order.begin(), order.end(), 0);
     cudaError_t e;
-    if ((e = cudaMalloc(&b->d_probs, sizeof(Prob2d) * count)) != cudaSuccess) return fail(e);
-    if ((e = cudaMalloc(&b->d_starts, sizeof(int) * starts.size())) != cudaSuccess) return fail(e);
-    if ((e = cudaMemcpy(b->d_probs, probs.data(), sizeof(Prob2d) * count,
-                        cudaMemcpyHostToDevice)) != cudaSuccess)
-        return fail(e);
-    if ((e = cudaMemcpy(b->d_starts, starts.data(), sizeof(int) * starts.size(),
-                        cudaMemcpyHostToDevice)) != cudaSuccess)
-        return fail(e);
+    if ((e = upload_work(*b, order, &b->d_probs, &b->d_starts)) != cudaSuccess) return fail(e);
+    for (int k = 0; k < 2; ++k) {
+        std::iota(order.begin(), order.end(), 0);
+        std::stable_sort(order.begin(), order.end(), [&](int i, int j) {
+            const Prob2d &x = b->probs[i], &y = b->probs[j];
+            return k == 0 ? std::max(x.W, x.H) > std::max(y.W, y.H) : x.nangles > y.nangles;
+        });
+        if ((e = upload_work(*b, order, &b->d_sorted[k], &b->d_sorted_starts[k])) != cudaSuccess)
+            return fail(e);
+    }
     *batch = b.release();
     return CG_OK;
 }
@@ -182,16 +222,17 @@ int cg_batch2d_forward(cg_batch2d *batch, void *stream) {
     CG_REQUIRE(guard.ok(), "cannot select the batch's device");
     int totals[kBatchStages];
     batch->active_totals(totals);
+    const bool all = batch->active == batch->count;
+    const Prob2d *probs = all ? batch->d_sorted[0] : batch->d_probs;
+    const int *starts = all ? batch->d_sorted_starts[0] : batch->d_starts;
     if (batch->fwd_algo == 1)
-        return launch_batch2d_fwd_tex(batch->d_probs, batch->probs, batch->active,
-                                      batch->d_starts + (batch->count + 1), totals[1],
+        return launch_batch2d_fwd_tex(probs, batch->probs, batch->active,
+                                      starts + (batch->count + 1), totals[1],
                                       (cudaStream_t)stream);
     if (batch->fwd_algo == 2)
-        return launch_batch2d_fwd_plans(batch->d_probs, batch->probs, batch->active,
-                                        batch->d_starts, totals, batch->count,
-                                        (cudaStream_t)stream);
-    return launch_batch2d(batch->d_probs, batch->d_starts, totals, batch->count, true,
-                          (cudaStream_t)stream);
+        return launch_batch2d_fwd_plans(probs, batch->probs, batch->active, starts, totals,
+                                        batch->count, (cudaStream_t)stream);
+    return launch_batch2d(probs, starts, totals, batch->count, true, (cudaStream_t)stream);
 }
 
 int cg_batch2d_set_active(cg_batch2d *batch, int active) {
@@ -246,8 +287,10 @@ int cg_batch2d_backward(cg_batch2d *batch, void *stream) {
     CG_REQUIRE(guard.ok(), "cannot select the batch's device");
     int totals[kBatchStages];
     batch->active_totals(totals);
-    return launch_batch2d(batch->d_probs, batch->d_starts, totals, batch->count, false,
-                          (cudaStream_t)stream);
+    const bool all = batch->active == batch->count;
+    return launch_batch2d(all ? batch->d_sorted[1] : batch->d_probs,
+                          all ? batch->d_sorted_starts[1] : batch->d_starts, totals, batch->count,
+                          false, (cudaStream_t)stream);
 }
 
 int cg_batch3d_create(cg_batch3d **batch, cg_plan3d *const *plans, float *const *volumes,
