@@ -161,6 +161,7 @@ int cg_batch2d_create(cg_batch2d **batch, cg_plan2d *const *plans, float *const 
         q.quadA = p.d_quadA, q.quadB = p.d_quadB;
         q.chunked = batch_chunked(p) ? 1 : 0;
         q.bwd_sym = p.bwd_sym;
+        q.bwd_per = bwd_group_views(p);
         int blocks[kBatchStages];
         batch_blocks(p, blocks);
         for (int st = 0; st < kBatchStages; ++st) {

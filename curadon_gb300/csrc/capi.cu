@@ -777,9 +777,9 @@ int forward2d_f32(cg_plan2d *plan, const float *volume, float *sinogram, cudaStr
 
 int backward2d_f32(cg_plan2d *plan, float *volume, const float *sinogram, cudaStream_t s) {
     if (plan->algo_bwd == 1) return launch_backward2d_tex(*plan, volume, sinogram, s);
+    if (plan->algo_bwd == 2) return launch_backward2d_smem(*plan, volume, sinogram, s);
     int rc = launch_relayout_sino2d(*plan, sinogram, s);
     if (rc) return rc;
-    if (plan->algo_bwd == 2) return launch_backward2d_smem(*plan, volume, s);
     return launch_backward2d(*plan, volume, s);
 }
 

@@ -156,6 +156,7 @@ struct Prob2d {
     float4 *quadA, *quadB;    // matched adjoint: the plan's quad accumulators
     int chunked;              // the batched "plans" forward runs the chunked kernel
     int bwd_sym;              // the plan's quarter-turn symmetry (Plan2d::bwd_sym)
+    int bwd_per;              // views summed at a time (bwd_group_views)
 };
 
 // Problem of a batched launch's block b: the last i with start[i] <= b
@@ -334,9 +335,12 @@ int launch_backward3d(const Plan3d &p, float *vol, const float *sino, cudaStream
 int launch_adjoint2d(Plan2d &p, float *vol, const float *sino, cudaStream_t s);
 int launch_adjoint3d(Plan3d &p, float *vol, const float *sino, cudaStream_t s);
 
-int launch_backward2d_smem(const Plan2d &p, float *vol, cudaStream_t s);
+// the staged backprojection (with the sinogram's re-layout where it reads it)
+int launch_backward2d_smem(const Plan2d &p, float *vol, const float *sino, cudaStream_t s);
 // blocks of the quarter-turn backprojection of a W x W image
 int sym_quadrant_blocks(int W);
+// views whose sum the staged backprojection adds to the volume at a time
+int bwd_group_views(const Plan2d &p);
 int sm_count();
 // rows: the chunked forward's compiled shape (kFwdChunkShapes: 443, 474, 484)
 int launch_forward2d_cslab(const Plan2d &p, float *sino, cudaStream_t s, int rows);

@@ -13,6 +13,8 @@
 // along y read layA, rays that advance along x read the transposed layB.
 // Interpolation is FP32 in registers (no texture unit); clamping a texel
 // index into the zero padding reproduces cudaAddressModeBorder.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <cfloat>
 #include <climits>
@@ -807,6 +809,31 @@ __global__ void __launch_bounds__(256)
 
 // ------------------------------------------------------------ backward, staged
 
+// Adds the parts of a cluster's CTAs (`count` sums each, a multiple of 32, at
+// the same place of every CTA's shared memory) to the volume in the order of
+// the CTAs: CTA `group` takes every gridDim.z-th run of 32 sums; at(e) is the
+// address of sum e's pixel, nullptr outside the image.
+template <class At>
+__device__ __forceinline__ void add_cluster_parts(float *part, int count, int group, float inv,
+                                                  At at) {
+    namespace cgr = cooperative_groups;
+    cgr::cluster_group cluster = cgr::this_cluster();
+    cluster.sync();
+    const int tid = threadIdx.y * blockDim.x + threadIdx.x;
+    const int groups = gridDim.z, lane = tid & 31, warps = (blockDim.x * blockDim.y) >> 5;
+    for (int run = (tid >> 5) * groups + group; run < count / 32; run += warps * groups) {
+        float *to = at(run * 32 + lane);
+        if (!to) continue;
+        float v = *to;
+        for (int g = 0; g < groups; ++g)
+            v = fmaf(*cluster.map_shared_rank(part + run * 32 + lane, g), inv, v);
+        *to = v;
+    }
+    cluster.sync();  // the parts stay until every CTA has read them
+}
+
+constexpr int kDirectGroups = 16;  // groups of views of the direct kernel at most
+constexpr int kClusterGroups = 8;  // and of a cluster
 constexpr int kSmRows = 8;    // pixels per thread, 8 rows apart: 32 x 64 tiles
 constexpr int kSmViews = 32;  // views staged per pass
 constexpr int kSmWin = 128;   // pairs of one view's row staged for a tile
@@ -837,13 +864,19 @@ constexpr int kSmWin = 128;   // pairs of one view's row staged for a tile
 // R: pixels per thread (rows 8 apart), so tiles of 32 x 8R pixels; every
 // pixel's sum runs over the views in the same order whatever R, so results
 // do not depend on it.
+// A pixel's views are summed in groups of `per` views (bwd_group_views): each
+// group's sum is added to the volume, one group after the other.  CLUSTER:
+// the CTAs of a cluster take one group each (`group`) and add their parts in
+// that order through distributed shared memory; otherwise the block takes the
+// groups in turn.  The results are the same bits.
 template <bool PK, bool MAGIC = false, int VU = 2, bool CPA = false, bool ABS = false,
-          bool MAPQ = false, bool BULK = false, int R = kSmRows>
+          bool MAPQ = false, bool BULK = false, int R = kSmRows, bool CLUSTER = false>
 __device__ __forceinline__ void bwd2d_smem_tile(float *__restrict__ vol,
                                                 const float2 *__restrict__ S,
                                                 const float4 *__restrict__ proj, int W, int H,
                                                 int det, int nangles, float sx, float sy, float ox,
-                                                float oy, float ds, int bx, int by) {
+                                                float oy, float ds, int bx, int by, int per,
+                                                int group = 0) {
     constexpr int kRow = BULK ? kSmWin + 2 : kSmWin;  // pairs per staged row
     static_assert(kRow * sizeof(float2) % 16 == 0, "bulk rows are multiples of 16 bytes");
     __shared__ __align__(16) float2 srow[kSmViews][kRow];
@@ -888,14 +921,35 @@ __device__ __forceinline__ void bwd2d_smem_tile(float *__restrict__ vol,
             mbar_fence_init();
         }
     }
-    // BULK: a wait that gives up stops the tile at the next group of views
+    // adds the group's sums to the volume and starts the next group
+    auto flush = [&]() {
+        if (x >= W) return;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int y = y0 + 8 * r;
+            float &a = (r & 1) ? acc2[r >> 1].y : acc2[r >> 1].x;
+            if (y < H) {
+                float &v = vol[(size_t)y * W + x];
+                v = fmaf(a, inv, v);
+            }
+            a = 0.f;
+        }
+    };
+    // BULK: a wait that gives up stops the tile at the next pass of views
     // (every thread learns it from the same barrier), so no further copy is
     // issued; before exit thread 0 waits, again bounded, for the copies it
     // has not seen complete.  The tile's results are then not to be trusted
     // and the give-up is counted for cg_wait_timeouts.
     int gave_up = 0;
-    for (int v0 = 0; v0 < nangles; v0 += kSmViews) {
-        const int nv = min(kSmViews, nangles - v0);
+    const int va = CLUSTER ? group * per : 0;
+    const int vb = CLUSTER ? min(va + per, nangles) : nangles;
+    int vgroup = va + per;  // end of the group being summed
+    for (int v0 = va; v0 < vb; v0 += kSmViews) {
+        const int nv = min(kSmViews, vb - v0);
+        if (!CLUSTER && v0 == vgroup) {
+            flush();
+            vgroup += per;
+        }
         if constexpr (BULK) {
             if (__syncthreads_or(gave_up)) break;
         } else {
@@ -1071,13 +1125,22 @@ __device__ __forceinline__ void bwd2d_smem_tile(float *__restrict__ vol,
             if (gave_up) mbar_wait(bar, phase, kWaitTries);
         }
     }
-    if (x < W) {
+    if constexpr (CLUSTER) {
+        // the parts lie in the CTAs' staged rows, which are no longer read
+        static_assert(sizeof(srow) >= sizeof(float) * 256 * R, "parts fit the staged rows");
+        float *part = reinterpret_cast<float *>(srow);
+        __syncthreads();
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const int y = y0 + 8 * r;
-            const float a = (r & 1) ? acc2[r >> 1].y : acc2[r >> 1].x;
-            if (y < H) vol[(size_t)y * W + x] += a * inv;
-        }
+        for (int r = 0; r < R; ++r)
+            part[r * 256 + tid] = (r & 1) ? acc2[r >> 1].y : acc2[r >> 1].x;
+        add_cluster_parts(part, 256 * R, group, inv, [&](int e) -> float * {
+            const int t = e & 255, tx = t & 31, ty = t >> 5;
+            const int px = xt + (MAPQ ? (ty & 3) * 8 + (tx & 7) : tx);
+            const int py = yt + (MAPQ ? (ty >> 2) * 4 + (tx >> 3) : ty) + 8 * (e >> 8);
+            return px < W && py < H ? vol + (size_t)py * W + px : nullptr;
+        });
+    } else {
+        flush();
     }
 }
 
@@ -1334,10 +1397,89 @@ template <int MINB, bool PK, bool MAGIC = false, int VU = 2, bool CPA = false, b
 __global__ void __launch_bounds__(256, MINB)
     k_bwd2d_smem(float *__restrict__ vol, const float2 *__restrict__ S,
                  const float4 *__restrict__ proj, int W, int H, int det, int nangles, float sx,
-                 float sy, float ox, float oy, float ds) {
+                 float sy, float ox, float oy, float ds, int per) {
     bwd2d_smem_tile<PK, MAGIC, VU, CPA, ABS, MAPQ, BULK, R>(vol, S, proj, W, H, det, nangles,
                                                             sx, sy, ox, oy, ds, blockIdx.x,
-                                                            blockIdx.y);
+                                                            blockIdx.y, per);
+}
+
+// Small images: no staging and no re-layout.  Each warp takes 8 x 8 pixels
+// (two per lane, four rows apart) and one group of views, the block's warps
+// the groups of the same pixels; the samples come from the sinogram itself
+// through L1, the pair's absolute-position form is taken on the fly in the
+// re-layout's operations, and the groups' sums are added in order, so the
+// results are those of the staged tiles bit for bit.
+template <int G>
+__global__ void __launch_bounds__(32 * G)
+    k_bwd2d_direct(float *__restrict__ vol, const float *__restrict__ sino,
+                   const float4 *__restrict__ proj, int W, int H, int det, int nangles, float sx,
+                   float sy, float ox, float oy, float ds, int per) {
+    __shared__ float4 sA[G][32], sB[G][32];
+    __shared__ float part[G][64];
+    const int lane = threadIdx.x, group = threadIdx.y, groups = blockDim.y;
+    const int x = blockIdx.x * 8 + (lane & 7), y0 = blockIdx.y * 8 + (lane >> 3);
+    const float ex = (float)W / 2.0f, ey = (float)H / 2.0f;
+    const int cq = det / 2;
+    const float edq = ((float)det / 2.0f - 0.5f) - (float)cq;
+    const float inv = __fdividef(1.0f, ds);
+    const float X = ((float)x - ex) * sx + ox + 0.5f;
+    const float2 Yr = make_float2(((float)y0 - ey) * sy + oy + 0.5f,
+                                  ((float)(y0 + 4) - ey) * sy + oy + 0.5f);
+    const float2 M2 = make_float2(12582912.0f, 12582912.0f), e2 = make_float2(edq, edq);
+    float2 acc = make_float2(0.f, 0.f);
+    const int va = group * per, vb = min(va + per, nangles);
+    for (int v0 = va; v0 < vb; v0 += 32) {
+        const int nv = min(32, vb - v0);
+        if (lane < nv) {
+            sA[group][lane] = proj[v0 + lane];
+            sB[group][lane] = proj[nangles + v0 + lane];
+        }
+        __syncwarp();
+        const float *row = sino + (size_t)v0 * det;
+#pragma unroll 1
+        for (int j = 0; j < nv; ++j, row += det) {
+            const float4 a = sA[group][j], b = sB[group][j];
+            const float A = fmaf(a.x, X, a.z), B = fmaf(b.x, X, b.z);
+            const float2 den = __ffma2_rn(make_float2(a.y, a.y), Yr, make_float2(A, A));
+            const float2 yi = __ffma2_rn(make_float2(b.y, b.y), Yr, make_float2(B, B));
+            const float2 w = make_float2(rcp_approx(den.x), rcp_approx(den.y));
+            const float2 ub = __ffma2_rn(w, yi, e2);
+            // floor by the round-down add (|ub| >= 2^22, infinities and NaN
+            // fall outside the row)
+            const float2 t = __fadd2_rd(ub, M2);
+            const int k0 = (int)(__float_as_uint(t.x) - 0x4B400000u) + cq;
+            const int k1 = (int)(__float_as_uint(t.y) - 0x4B400000u) + cq;
+            const float s00 = (unsigned)k0 < (unsigned)det ? __ldg(row + k0) : 0.f;
+            const float s01 = (unsigned)(k0 + 1) < (unsigned)det ? __ldg(row + k0 + 1) : 0.f;
+            const float s10 = (unsigned)k1 < (unsigned)det ? __ldg(row + k1) : 0.f;
+            const float s11 = (unsigned)(k1 + 1) < (unsigned)det ? __ldg(row + k1 + 1) : 0.f;
+            const float d0 = s01 - s00, d1 = s11 - s10;
+            const float g0 = fmaf(-(float)(k0 - cq), d0, s00), g1 = fmaf(-(float)(k1 - cq), d1, s10);
+            const float2 v = make_float2(fmaf(ub.x, d0, g0), fmaf(ub.y, d1, g1));
+            acc = __ffma2_rn(v, w, acc);
+        }
+        __syncwarp();
+    }
+    part[group][lane] = acc.x, part[group][32 + lane] = acc.y;
+    __syncthreads();
+    for (int e = group * 32 + lane; e < 64; e += groups * 32) {
+        const int px = blockIdx.x * 8 + (e & 7), py = blockIdx.y * 8 + (e >> 3);
+        if (px >= W || py >= H) continue;
+        float v = vol[(size_t)py * W + px];
+        for (int g = 0; g < groups; ++g) v = fmaf(part[g][e], inv, v);
+        vol[(size_t)py * W + px] = v;
+    }
+}
+
+// The same tiles with the views in groups: CTA z of a cluster takes group z.
+template <int MINB>
+__global__ void __launch_bounds__(256, MINB)
+    k_bwd2d_cluster(float *__restrict__ vol, const float2 *__restrict__ S,
+                    const float4 *__restrict__ proj, int W, int H, int det, int nangles, float sx,
+                    float sy, float ox, float oy, float ds, int per) {
+    bwd2d_smem_tile<true, true, 4, true, true, true, true, kSmRows, true>(
+        vol, S, proj, W, H, det, nangles, sx, sy, ox, oy, ds, blockIdx.x, blockIdx.y, per,
+        blockIdx.z);
 }
 
 }  // namespace
@@ -1416,7 +1558,8 @@ __global__ void __launch_bounds__(256, 4)
     const int gx = (q.W + 31) / 32;
     bwd2d_smem_tile<true, true, 4, true, true, true, true>(q.vol, q.sinoP, q.bproj, q.W, q.H,
                                                            q.det, q.nangles, q.sx, q.sy, q.ox,
-                                                           q.oy, q.ds, local % gx, local / gx);
+                                                           q.oy, q.ds, local % gx, local / gx,
+                                                           q.bwd_per);
 }
 
 // The quarter-turn symmetric tile of the single-problem default for the
@@ -1559,44 +1702,100 @@ int sm_count() {
 
 int sym_quadrant_blocks(int W) { return ceil_div(W / 2, 32) * ceil_div(W / 2, 8 * kSymR); }
 
-int launch_backward2d_smem(const Plan2d &p, float *vol, cudaStream_t s) {
+// The direct kernel for few (pixel, view) pairs: staged tiles are then too few
+// to fill the SMs, and each CTA of a cluster of 8 is a chain of ceil(passes /
+// 8) passes of about 5 us, where the direct kernel takes 8 us and 0.7 us per
+// M pairs; beyond, shared windows cost less per pair.  A single pass (32 views
+// or fewer) stays staged: one warp per pixel patch would walk it alone.
+// Clusters / direct, us in a CUDA graph: 64^2 x 360 18.8 / 8.8 (no clusters
+// 59), 256^2 x 60 11.7 / 9.3, 128^2 x 720 25.8 / 17.9, 200^2 x 300 (12 M) 19.1 /
+// 19.1, 256^2 x 256 (16.8 M) 14.5 / 20.3, 256^2 x 300 (19.7 M) 22.5 / 22.7;
+// one pass 256^2 x 31 7.7 / 9.0.
+static bool bwd_direct(const Plan2d &p) {
+    const int passes = ceil_div(p.nangles, kSmViews);
+    return !p.bwd_sym && passes > 1 &&
+           (double)p.W * p.H * p.nangles <= 6.5e6 * ceil_div(passes, kClusterGroups);
+}
+
+// Views summed at a time: nangles (one sum), or groups of them, a multiple of
+// the 32 views of a staged pass, for as many warps (direct kernel) or CTAs of a
+// cluster to share a tile's views.  The count of groups that gives the SMs the
+// most even load: the fullest SM has ceil(blocks / SMs) blocks of (passes +
+// 0.3 for the start and the end), and fewer than three resident blocks (five
+// of clusters, which do not fill every slot) leave it waiting on latency.
+// One group / the rule's, us: 512^2 x 512 116.8 / 68.5, 640^2 x 640 223 / 113,
+// 768^2 x 768 311 / 184, 1024^2 x 1024 490 / 408, 1280^2 x 1280 895 / 771,
+// 2048^2 x 2048 (no quarter turns) 3143 / 2915; 2048^2 x 360 564 and 1024^2 x
+// 90 52.5 keep one (eight: 604, 53.6).  The quarter-turn kernel keeps one: its
+// blocks are already even (2048^2 2672, two groups 2740).
+int bwd_group_views(const Plan2d &p) {
+    const int passes = ceil_div(p.nangles, kSmViews);
+    if (bwd_direct(p)) return kSmViews * ceil_div(passes, kDirectGroups);
+    if (p.bwd_sym) return p.nangles;
+    const long long tiles = (long long)ceil_div(p.W, 32) * ceil_div(p.H, 8 * kSmRows);
+    const long long sms = sm_count();
+    int best = passes;
+    double best_time = 0.0;
+    for (int g = 1; g <= kClusterGroups; ++g) {
+        const int per = ceil_div(passes, g);
+        const long long blocks = tiles * ceil_div(passes, per);
+        const double time = (double)std::max((blocks + sms - 1) / sms, g == 1 ? 3LL : 5LL) * (per + 0.3);
+        if (g == 1 || time < best_time) best = per, best_time = time;
+    }
+    return best >= passes ? p.nangles : best * kSmViews;
+}
+
+int launch_backward2d_smem(const Plan2d &p, float *vol, const float *sino, cudaStream_t s) {
+    const int per = bwd_group_views(p), groups = ceil_div(p.nangles, per);
+    auto go = [&](auto kernel, dim3 grid, dim3 block, unsigned cluster, auto... args) -> int {
+        cudaLaunchConfig_t c{};
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = at[0].val.clusterDim.y = 1, at[0].val.clusterDim.z = cluster;
+        c.gridDim = grid, c.blockDim = block, c.stream = s, c.attrs = at;
+        c.numAttrs = cluster > 1 ? 1 : 0;
+        CG_TRY_CUDA(cudaLaunchKernelEx(&c, kernel, vol, args...));
+        return CG_OK;
+    };
+    const bool standard = p.bwd_min_blocks == 68;
+    if (standard && bwd_direct(p))
+        return go(groups > 4 ? k_bwd2d_direct<kDirectGroups> : k_bwd2d_direct<4>,
+                  dim3(ceil_div(p.W, 8), ceil_div(p.H, 8)), dim3(32, groups), 1, sino, (const float4 *)p.d_bproj, p.W, p.H, p.det, p.nangles, p.sx, p.sy, p.ox,
+                  p.oy, p.ds, per);
+    if (int rc = launch_relayout_sino2d(p, sino, s)) return rc;
     if (p.bwd_sym != 0) {
         // the first quadrant's tiles, each with its three turned copies
         const int half = p.W / 2;
-        const dim3 grid(ceil_div(half, 32), ceil_div(half, 8 * kSymR));
-        k_bwd2d_sym<4><<<grid, dim3(32, 8), 0, s>>>(vol, p.d_sinoP, p.d_bproj, p.W, p.det,
-                                                 p.nangles, p.sx, p.ox, p.ds, p.bwd_sym);
-        CG_TRY_CUDA(cudaGetLastError());
-        return CG_OK;
+        return go(k_bwd2d_sym<4>, dim3(ceil_div(half, 32), ceil_div(half, 8 * kSymR)), dim3(32, 8), 1,
+                  (const float2 *)p.d_sinoP, (const float4 *)p.d_bproj, p.W, p.det, p.nangles, p.sx,
+                  p.ox, p.ds, p.bwd_sym);
     }
     // tiles of 32 x 64 pixels; an image whose tiles would not give every SM
     // two blocks takes 32 x 16-pixel tiles (two pixels per thread) instead,
-    // four times the blocks, the same sums
-    const bool small = (long long)ceil_div(p.W, 32) * ceil_div(p.H, 8 * kSmRows) < 2LL * sm_count();
-    const dim3 grid(ceil_div(p.W, 32), ceil_div(p.H, 8 * (small ? 2 : kSmRows)));
-    auto go = [&](auto kernel) {
-        kernel<<<grid, dim3(32, 8), 0, s>>>(vol, p.d_sinoP, p.d_bproj, p.W, p.H, p.det,
-                                            p.nangles, p.sx, p.sy, p.ox, p.oy, p.ds);
+    // four times the blocks, the same sums (unless clusters fill the SMs)
+    const bool cluster = standard && groups > 1;
+    const bool small = !cluster && (long long)ceil_div(p.W, 32) * ceil_div(p.H, 8 * kSmRows) < 2LL * sm_count();
+    auto tile = [&](auto kernel) {
+        const unsigned z = cluster ? groups : 1;
+        return go(kernel, dim3(ceil_div(p.W, 32), ceil_div(p.H, 8 * (small ? 2 : kSmRows)), z),
+                  dim3(32, 8), z, (const float2 *)p.d_sinoP, (const float4 *)p.d_bproj, p.W, p.H,
+                  p.det, p.nangles, p.sx, p.sy, p.ox, p.oy, p.ds, per);
     };
+    if (cluster) return tile(k_bwd2d_cluster<4>);
     // the default (68) and the autotuner's other candidates (48: the same
     // staged pair by pair with cp.async; 27: (t, d) pairs, 32 x 1-pixel warps,
     // view loop unrolled twice)
     switch (p.bwd_min_blocks) {
         case 27:
-            small ? go(k_bwd2d_smem<4, true, true, 2, true, false, false, false, 2>)
-                  : go(k_bwd2d_smem<4, true, true, 2, true>);
-            break;
+            return small ? tile(k_bwd2d_smem<4, true, true, 2, true, false, false, false, 2>)
+                         : tile(k_bwd2d_smem<4, true, true, 2, true>);
         case 48:
-            small ? go(k_bwd2d_smem<4, true, true, 4, true, true, true, false, 2>)
-                  : go(k_bwd2d_smem<4, true, true, 4, true, true, true>);
-            break;
+            return small ? tile(k_bwd2d_smem<4, true, true, 4, true, true, true, false, 2>)
+                         : tile(k_bwd2d_smem<4, true, true, 4, true, true, true>);
         default:
-            small ? go(k_bwd2d_smem<4, true, true, 4, true, true, true, true, 2>)
-                  : go(k_bwd2d_smem<4, true, true, 4, true, true, true, true>);
-            break;
+            return small ? tile(k_bwd2d_smem<4, true, true, 4, true, true, true, true, 2>)
+                         : tile(k_bwd2d_smem<4, true, true, 4, true, true, true, true>);
     }
-    CG_TRY_CUDA(cudaGetLastError());
-    return CG_OK;
 }
 
 int launch_backward2d(const Plan2d &p, float *vol, cudaStream_t s) {
