@@ -3,7 +3,7 @@
 scale by pi / (2 nangles), backproject.
 
 The filtering runs in the sm_103a kernel behind ``cg_filter_rows`` as a
-direct circular convolution with h = Re(IDFT(fftshift(w))), which equals the
+circular convolution with h = Re(IDFT(fftshift(w))), which equals the
 reference's ``_apply_filter`` (DFT of each row times fftshift(w), real part of
 the inverse DFT) exactly in exact arithmetic.
 """
