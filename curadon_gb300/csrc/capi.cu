@@ -73,7 +73,7 @@ bool listed(const int (&list)[N], int v) {
 // from CURADON_GB300_ALGO: comma-separated key=value tokens, e.g.
 // "fwd2d=tex,bwd2d_minb=48".  Keys: fwd2d = alu | tex | cslab |
 // cslab<443 | 474 | 484>; fwd2d_bundle = small | large (the chunked forward's
-// bundles); bwd2d = alu | tex | smem; bwd2d_minb = 27 | 48 | 68
+// bundles); fwd2d_march = off (the register forward ray by ray); bwd2d = alu | tex | smem; bwd2d_minb = 27 | 48 | 68
 // (staged backprojector variants); adj2d = pair | quad; fwd3d = alu | tex3 |
 // quad | mixed; fwd3d_tex = 0..8 (texture warps of 8 in the mixed forward);
 // fwd3d_unroll = 1 | 2 (samples per iteration of the quad / mixed forward);
@@ -111,6 +111,7 @@ void apply_algo_env(Plan2d *p2, Plan3d *p3) {
                     if (val == "cslab" + std::to_string(k)) p2->fwd_chunk_rows = k;
             }
         }
+        if (p2 && key == "fwd2d_march" && val == "off") p2->fwd_march = false;
         if (p2 && key == "fwd2d_bundle") {
             if (val == "small") p2->fwd_bundle = -1;
             if (val == "large") p2->fwd_bundle = 1;

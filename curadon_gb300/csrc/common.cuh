@@ -120,6 +120,9 @@ struct Plan2d {
     // one (CURADON_GB300_ALGO fwd2d_bundle=small / large)
     double view_step = 0;
     int fwd_bundle = 0;
+    // the register forward in bundles (CURADON_GB300_ALGO fwd2d_march=off: ray
+    // by ray, the same bits)
+    bool fwd_march = true;
     // staged backprojector's variant: 68 (default: packed FP32 row pairs,
     // floor by FP32 adds, window rows by bulk copies, absolute-position
     // pairs, 8 x 4-pixel warps), 48 (the same staged pair by pair with
@@ -204,7 +207,9 @@ constexpr int kBatch3dStages = 9;
 // absolute-position re-layout and chunked bundles (chunked problems) and
 // texture rays (the others), and the backprojection over the quarter-turn
 // symmetry (problems whose plan has it; stage 3 holds the others).
-constexpr int kBatchStages = 11;
+// Stages 11 and 12 are the register forward's: bundles, and rays for the
+// problems that have none.
+constexpr int kBatchStages = 13;
 // chunked-forward shape the batched "plans" forward compiles
 constexpr int kBatchChunkShape = 484;
 

@@ -19,6 +19,7 @@
 #include <cfloat>
 #include <climits>
 #include <cmath>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -365,7 +366,7 @@ constexpr int kWaitTries = 1 << 22;
 // One bundle (bx: cells, by: views, bz: ray class) of the chunked forward;
 // the kernels below run it over a grid (one problem) or a work list (many).
 template <int K, int S, int T, bool PK, bool REUSE = false, int VS = 1, int NG = kCs2G,
-          int MB = 0, int MAP = 0, bool ABS = false, bool TMA = false>
+          int MB = 0, int MAP = 0, bool ABS = false, bool TMA = false, bool MARCH = false>
 __device__ __forceinline__ void cslab_bundle(const float2 *__restrict__ layA,
                                              const float2 *__restrict__ layB,
                                              float *__restrict__ sino,
@@ -437,6 +438,7 @@ __device__ __forceinline__ void cslab_bundle(const float2 *__restrict__ layA,
     RowAcc<PK> acc[GV];
     int rlo[GV], len[GV];
     int my_min = INT_MAX, my_max = INT_MIN;
+    unsigned ups = 0, downs = 0, alone = 0;
 #pragma unroll
     for (int g = 0; g < GV; ++g) {
         const int view = v0 + bview(g);
@@ -448,12 +450,34 @@ __device__ __forceinline__ void cslab_bundle(const float2 *__restrict__ layA,
         const int iq = (int)fminf(fmaxf(floorf(r.q), -(float)kPad), (float)qmax);
         const int n = min(r.n, r.sq > 0 ? qmax - iq + 1 : iq + kPad + 1);
         if (n <= 0) continue;
+        if constexpr (MARCH) {
+            V[g] = r.vp, p[g] = r.p, rlo[g] = iq, len[g] = n;
+            (r.sq > 0 ? ups : downs) |= 1u << g;
+            continue;
+        }
         const int lo = r.sq > 0 ? iq : iq - (n - 1);
         V[g] = r.sq > 0 ? r.vp : -r.vp;
         p[g] = (r.sq > 0 ? r.p : fmaf((float)(n - 1), r.vp, r.p)) - pc;
         rlo[g] = lo, len[g] = n;
         my_min = min(my_min, lo), my_max = max(my_max, lo + n - 1);
     }
+    // MARCH: the bundle walks the rows the way its rays do (desc: m = -row
+    // counts them); a ray that goes against the others marches on its own
+    bool desc = false;
+    if constexpr (MARCH) {
+        const bool any_up = __syncthreads_or(ups != 0), any_down = __syncthreads_or(downs != 0);
+        desc = any_down && !any_up;
+        alone = desc ? 0u : downs;
+#pragma unroll
+        for (int g = 0; g < GV; ++g) {
+            if ((alone >> g) & 1u) len[g] = 0;
+            if (len[g] == 0) continue;
+            if (desc) rlo[g] = -rlo[g];
+            my_min = min(my_min, rlo[g]), my_max = max(my_max, rlo[g] + len[g] - 1);
+        }
+    }
+    // lowest row of the chunk that starts at m
+    auto low_row = [&](int m) { return MARCH && desc ? -(m + K - 1) : m; };
     if (my_min <= my_max) {
         atomicMin(&s_rmin, my_min);
         atomicMax(&s_rmax, my_max);
@@ -463,7 +487,7 @@ __device__ __forceinline__ void cslab_bundle(const float2 *__restrict__ layA,
     const int nch = rmin <= rmax ? (rmax - rmin) / K + 1 : 0;
     {
         for (int ci = threadIdx.x; ci < min(nch, kCs2MaxChunks); ci += NT) {
-            const float ra = (float)(rmin + ci * K), rb = ra + (float)K;
+            const float ra = (float)low_row(rmin + ci * K), rb = ra + (float)K;
             float lo = FLT_MAX, hi = -FLT_MAX;
 #pragma unroll
             for (int c = 0; c < 2 * NG; ++c) {
@@ -489,10 +513,10 @@ __device__ __forceinline__ void cslab_bundle(const float2 *__restrict__ layA,
     auto stage = [&](int ci, int buf) {
         const int win = ci < kCs2MaxChunks ? s_win[ci] : -1;
         if (win < 0) return;
-        const int c0 = win >> 16, wx = win & 0xffff, r0 = rmin + ci * K;
+        const int c0 = win >> 16, wx = win & 0xffff, r0 = low_row(rmin + ci * K);
         float2 *base = cwin + buf * kBuf;
         for (int row = warp; row <= K; row += NT / 32) {
-            const int q = min(r0 + row, qmax + 1);
+            const int q = MARCH ? max(min(r0 + row, qmax + 1), -kPad) : min(r0 + row, qmax + 1);
             const float2 *src = lay + (size_t)(q + kPad) * pitch + c0;
             float2 *dst = base + row * S;
             for (int c = 2 * lane; c < wx; c += 64) {
@@ -511,7 +535,7 @@ __device__ __forceinline__ void cslab_bundle(const float2 *__restrict__ layA,
     auto stage_tma = [&](int ci, int buf) {
         const int win = ci < kCs2MaxChunks ? s_win[ci] : -1;
         if (win < 0 || warp != 0) return;
-        const int c0 = win >> 16, wx = win & 0xffff, r0 = rmin + ci * K;
+        const int c0 = win >> 16, wx = win & 0xffff, r0 = low_row(rmin + ci * K);
         const unsigned bar = bar0 + 8u * (unsigned)buf;
         const unsigned row_bytes = (unsigned)wx * (unsigned)sizeof(float2);
         if (lane == 0) {
@@ -521,7 +545,7 @@ __device__ __forceinline__ void cslab_bundle(const float2 *__restrict__ layA,
         __syncwarp();
         const unsigned base = (unsigned)__cvta_generic_to_shared(cwin + buf * kBuf);
         for (int row = lane; row <= K; row += 32) {
-            const int q = min(r0 + row, qmax + 1);
+            const int q = MARCH ? max(min(r0 + row, qmax + 1), -kPad) : min(r0 + row, qmax + 1);
             bulk_copy_g2s(base + (unsigned)(row * S) * (unsigned)sizeof(float2),
                           lay + (size_t)(q + kPad) * pitch + c0, row_bytes, bar);
         }
@@ -579,6 +603,9 @@ __device__ __forceinline__ void cslab_bundle(const float2 *__restrict__ layA,
             const int c0 = (win >> 16) - kPad, wx = win & 0xffff;
             const unsigned cmax = (unsigned)(wx - 1);
             const float2 *b0 = cwin + (ci & 1) * kBuf;
+            // buffer row of the chunk's k-th row
+            auto samples = [&](auto down) {
+                auto at = [&](int k) { return decltype(down)::value ? K - 1 - k : k; };
 #pragma unroll
             for (int g = 0; g < GV; ++g) {
                 const int rel = r0 - rlo[g];
@@ -592,10 +619,10 @@ __device__ __forceinline__ void cslab_bundle(const float2 *__restrict__ layA,
                     for (int k = 0; k < K; ++k) {
                         float fp;
                         const unsigned c = cs_column<ABS>(p[g], c0 - ic, cmax, fp);
-                        const float2 hi = b0[(k + 1) * S + c];
+                        const float2 hi = b0[(at(k) + 1) * S + c];
                         float2 lo;
                         if (REUSE && c == c_prev) lo = hi_prev;
-                        else lo = b0[k * S + c];
+                        else lo = b0[at(k) * S + c];
                         acc[g].add(fp, lo, hi);
                         if (REUSE) c_prev = c, hi_prev = hi;
                         p[g] += V[g];
@@ -606,13 +633,16 @@ __device__ __forceinline__ void cslab_bundle(const float2 *__restrict__ layA,
                         if ((unsigned)(rel + k) < (unsigned)len[g]) {
                             float fp;
                             const unsigned c = cs_column<ABS>(p[g], c0 - ic, cmax, fp);
-                            const float2 lo = b0[k * S + c], hi = b0[(k + 1) * S + c];
+                            const float2 lo = b0[at(k) * S + c], hi = b0[(at(k) + 1) * S + c];
                             acc[g].add(fp, lo, hi);
                             p[g] += V[g];
                         }
                     }
                 }
             }
+            };
+            if (MARCH && desc) samples(std::true_type{});
+            else samples(std::false_type{});
         } else {
             // a window wider than the buffer: the samples from global memory,
             // GR rows of a ray at a time with their loads issued together (one
@@ -625,14 +655,15 @@ __device__ __forceinline__ void cslab_bundle(const float2 *__restrict__ layA,
 #pragma unroll
             for (int g = 0; g < GV; ++g) {
                 const int ra = max(r0, rlo[g]), rb = min(r0 + K, rlo[g] + len[g]);
-                for (int rg = ra; rg < rb; rg += GR) {
+                for (int rg = ra; rg < rb; rg += GR) {  // (m, like r0)
                     float fp[GR];
                     float2 lo[GR], hi[GR];
 #pragma unroll
                     for (int k = 0; k < GR; ++k) {
                         // rows past the ray's last are loaded from it and dropped
                         const unsigned c = cs_column<ABS>(p[g], -kPad - ic, gcap, fp[k]);
-                        const float2 *rowp = lay + (size_t)(min(rg + k, rb - 1) + kPad) * pitch + c;
+                        const int m = min(rg + k, rb - 1);
+                        const float2 *rowp = lay + (size_t)((MARCH && desc ? -m : m) + kPad) * pitch + c;
                         lo[k] = __ldg(rowp), hi[k] = __ldg(rowp + pitch);
                         if (rg + k < rb) p[g] += V[g];
                     }
@@ -656,6 +687,10 @@ __device__ __forceinline__ void cslab_bundle(const float2 *__restrict__ layA,
     for (int g = 0; g < GV; ++g) {
         const int view = v0 + bview(g);
         if (view >= nangles || u >= det) continue;
+        if (MARCH && ((alone >> g) & 1u)) {
+            fwd2d_ray(layA, layB, sino, tsrc, tu0, tdu, W, H, det, nangles, sx, sy, pa, pb, u, view);
+            continue;
+        }
         FanRay r;
         float out;
         if (!fan_ray(tsrc[view], tu0[view], tdu[view], u, W, H, sx, sy, r)) {
@@ -688,6 +723,37 @@ __global__ void __launch_bounds__(T * VS, MB)
 // each): 8 views x 128 cells (three blocks of 256 threads per SM) and 4 views
 // x 64 cells (five blocks of 128).
 constexpr int kCsRows = 16, kCsCols = 256, kCsSmallCols = 144;
+// The register forward (k_fwd2d) from shared windows: bundles of 4 views x 64
+// cells whose rays take their samples in their own order and in that kernel's
+// operations, so the same bits.  k_fwd2d's two 8-byte loads of a sample go
+// through L1 one warp at a time; here they come from a window that 256 rays
+// share.  k_fwd2d / this, us in a CUDA graph: 64^2 x 360 views 23.5 / 20.7,
+// 256^2 x 256 90 / 54, 513^2 x 437 239 / 155, 1024^2 x 1024 1334 / 833, 2048^2
+// x 1024 5242 / 2924 (8 views x 128 cells: 30.8, 97, 215, 975, 2861).
+__device__ __forceinline__ void march_bundle(const float2 *layA, const float2 *layB, float *sino,
+                                             const float2 *tsrc, const float2 *tu0,
+                                             const float2 *tdu, int W, int H, int det, int nangles,
+                                             float sx, float sy, int pa, int pb, int bx, int by,
+                                             int bz) {
+    cslab_bundle<kCsRows, kCsSmallCols, 64, false, false, 2, 4, 5, 2, false, true, true>(
+        layA, layB, sino, tsrc, tu0, tdu, W, H, det, nangles, sx, sy, pa, pb, bx, by, bz);
+}
+
+__global__ void __launch_bounds__(128, 5)
+    k_fwd2d_march(const float2 *__restrict__ layA, const float2 *__restrict__ layB,
+                  float *__restrict__ sino, const float2 *__restrict__ tsrc,
+                  const float2 *__restrict__ tu0, const float2 *__restrict__ tdu, int W, int H,
+                  int det, int nangles, float sx, float sy, int pa, int pb) {
+    march_bundle(layA, layB, sino, tsrc, tu0, tdu, W, H, det, nangles, sx, sy, pa, pb, blockIdx.x,
+                 blockIdx.y, blockIdx.z);
+}
+
+// Its window table packs columns in 16 bits, its grid 4 views per row.
+static bool marches(const Plan2d &p) {
+    return p.fwd_march && std::max(p.pitchA(), p.pitchB()) < 32768 &&
+           ceil_div(p.nangles, 4) <= 65535;
+}
+
 static size_t cslab_smem(int stride) { return 2 * sizeof(float2) * (kCsRows + 1) * stride; }
 
 // Which bundle the chunked forward takes (the sums are the same bits).  The
@@ -1527,6 +1593,19 @@ __global__ void __launch_bounds__(256, 3)
         q.pb, local % gx, (local / gx) % gy, local / (gx * gy));
 }
 
+// The register forward of the problems that march in bundles (stage 11) and,
+// below, of the others ray by ray (stage 12).
+__global__ void __launch_bounds__(128, 5)
+    k_batch_fwd2d_march(const Prob2d *__restrict__ probs, const int *__restrict__ start,
+                        int count) {
+    const int i = batch_problem(start, count, blockIdx.x);
+    const Prob2d &q = probs[i];
+    const int local = blockIdx.x - start[i];
+    const int gx = (q.det + 63) / 64, gy = (q.nangles + 3) / 4;
+    march_bundle(q.layA, q.layB, q.sino, q.src, q.u0, q.du, q.W, q.H, q.det, q.nangles, q.sx, q.sy,
+                 q.pa, q.pb, local % gx, (local / gx) % gy, local / (gx * gy));
+}
+
 __global__ void __launch_bounds__(256)
     k_batch_fwd2d(const Prob2d *__restrict__ probs, const int *__restrict__ start, int count) {
     const int i = batch_problem(start, count, blockIdx.x);
@@ -1598,6 +1677,8 @@ void batch_blocks(const Plan2d &p, int blocks[kBatchStages]) {
     blocks[7] = chunked ? blocks[0] : 0;
     blocks[8] = chunked ? ceil_div(p.det, 128) * ceil_div(p.nangles, 8) * 2 : 0;
     blocks[9] = chunked ? 0 : blocks[1];
+    blocks[11] = marches(p) ? ceil_div(p.det, 64) * ceil_div(p.nangles, 4) * 2 : 0;
+    blocks[12] = marches(p) ? 0 : blocks[1];
 }
 
 bool batch_chunked(const Plan2d &p) {
@@ -1628,7 +1709,15 @@ int launch_batch2d(const Prob2d *probs, const int *starts, const int totals[kBat
     if (forward) {
         k_batch_relayout2d<<<totals[0], tile, 0, s>>>(probs, starts, count);
         CG_TRY_CUDA(cudaGetLastError());
-        k_batch_fwd2d<<<totals[1], tile, 0, s>>>(probs, starts + (count + 1), count);
+        if (totals[11] > 0) {
+            const size_t smem = cslab_smem(kCsSmallCols);
+            if (int rc = ensure_smem_attr((const void *)k_batch_fwd2d_march, (int)smem)) return rc;
+            k_batch_fwd2d_march<<<totals[11], 128, smem, s>>>(probs, starts + 11 * (count + 1),
+                                                              count);
+            CG_TRY_CUDA(cudaGetLastError());
+        }
+        if (totals[12] > 0)
+            k_batch_fwd2d<<<totals[12], tile, 0, s>>>(probs, starts + 12 * (count + 1), count);
     } else {
         k_batch_relayout_sino2d<<<totals[2], 256, 0, s>>>(probs, starts + 2 * (count + 1), count);
         CG_TRY_CUDA(cudaGetLastError());
@@ -1667,6 +1756,16 @@ int launch_relayout2d(const Plan2d &p, const float *vol, cudaStream_t s) {
 }
 
 int launch_forward2d(const Plan2d &p, float *sino, cudaStream_t s) {
+    if (marches(p)) {
+        const size_t smem = cslab_smem(kCsSmallCols);
+        if (int rc = ensure_smem_attr((const void *)k_fwd2d_march, (int)smem)) return rc;
+        const dim3 grid(ceil_div(p.det, 64), ceil_div(p.nangles, 4), 2);
+        k_fwd2d_march<<<grid, 128, smem, s>>>(p.d_layA, p.d_layB, sino, p.d_src, p.d_u0, p.d_du,
+                                              p.W, p.H, p.det, p.nangles, p.sx, p.sy, p.pitchA(),
+                                              p.pitchB());
+        CG_TRY_CUDA(cudaGetLastError());
+        return CG_OK;
+    }
     dim3 block(p.fwd_bx, p.fwd_by);
     dim3 grid(ceil_div(p.det, p.fwd_bx), ceil_div(p.nangles, p.fwd_by));
     if (grid.y > 65535) return set_error(CG_ERR_INVALID, "too many views for one launch");

@@ -1,0 +1,47 @@
+"""The 2D register forward in bundles takes every ray's samples in the ray's own
+order and in the ray-by-ray kernel's operations: equal bits, alone and in a
+batch, where bundles have edges (64 cells, 4 views), rays of one bundle go both
+ways or the source lies close to (or inside) the image."""
+import numpy as np
+import pytest
+import torch
+
+from curadon_gb300 import FanGeometry, FanVecGeometry, forward
+from curadon_gb300.backend import forward_2d
+from curadon_gb300.batch import Batch2d
+from curadon_gb300.phantom import fan_config
+
+pytestmark = pytest.mark.gpu
+
+
+def geometries():
+    for n, views, det in ((33, 7, 50), (64, 3, 63), (64, 4, 64), (100, 5, 65), (257, 37, 364),
+                          (1024, 21, 1449)):
+        yield f"{n}", FanGeometry(**fan_config(n, views, det))
+    for dso, dsd, ds in ((80, 100, 2.0), (66, 400, 30.0), (30, 60, 3.0)):  # wide; inside
+        yield f"wide {dso}", FanGeometry(**fan_config(100, 90, 211, ds, dso, dsd))
+    g = dict(fan_config(48, 37, 70, 1.3, 90.0, 150.0), vol_shape=(48, 60), vol_spacing=(0.9, 1.2),
+             vol_offset=(2.0, -3.0), det_offset=1.5)
+    yield "offsets", FanGeometry(**g)
+    g = fan_config(300, 77)
+    v = np.asarray(FanGeometry(**g).to_vec())
+    v[:, 4:] *= g["det_spacing"]
+    v[::2] = np.concatenate([v[::2, :4] * [-1, -1, -1, -1], v[::2, 4:]], axis=1)  # both ways
+    yield "vectors", FanVecGeometry((300, 200), g["det_shape"], v)
+
+
+@pytest.mark.parametrize("name,geom", [pytest.param(n, g, id=n) for n, g in geometries()])
+def test_bundled_register_forward(cuda_device, monkeypatch, name, geom):
+    gen = torch.Generator(device=cuda_device).manual_seed(len(name))
+    vol = torch.rand(tuple(int(v) for v in geom.vol_shape), device=cuda_device, generator=gen)
+    alone = torch.full(geom.sinogram_shape(), -1.0, device=cuda_device)
+    batched, rays = torch.full_like(alone, -2.0), torch.full_like(alone, -3.0)
+    forward(vol, alone, geom, exact=True)
+    Batch2d([geom], [vol], [batched], forward="registers").forward()
+    monkeypatch.setenv("CURADON_GB300_ALGO", "fwd2d=alu,fwd2d_march=off")
+    plan = geom._make_plan()
+    monkeypatch.delenv("CURADON_GB300_ALGO")
+    forward_2d(vol, rays, plan)
+    torch.cuda.synchronize()
+    assert torch.equal(alone, rays)
+    assert torch.equal(batched, rays)
