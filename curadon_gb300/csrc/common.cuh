@@ -349,6 +349,8 @@ int bwd_group_views(const Plan2d &p);
 int sm_count();
 // rows: the chunked forward's compiled shape (kFwdChunkShapes: 443, 474, 484)
 int launch_forward2d_cslab(const Plan2d &p, float *sino, cudaStream_t s, int rows);
+// blocks of the texture forward
+int tex_blocks(const Plan2d &p);
 // The plan's 2D volume texture array and object (allocated once).
 int ensure_vol_texture(Plan2d &p);
 // the first `active` problems of a batch (the work list's blocks [0, total))

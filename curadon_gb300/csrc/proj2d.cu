@@ -1660,7 +1660,7 @@ __global__ void __launch_bounds__(256, 4)
 // single-problem kernels above).
 void batch_blocks(const Plan2d &p, int blocks[kBatchStages]) {
     blocks[0] = ceil_div(p.W + 2 * kPad, kTile) * ceil_div(p.H + 2 * kPad, kTile);
-    blocks[1] = ceil_div(p.det, 32) * ceil_div(p.nangles, 8);
+    blocks[1] = tex_blocks(p);
     blocks[2] = (int)ceil_div((long long)p.pitchS() * p.nangles, 256);
     blocks[3] = p.bwd_sym ? 0 : ceil_div(p.W, 32) * ceil_div(p.H, 8 * kSmRows);
     blocks[10] = p.bwd_sym ? ceil_div(p.W / 2, 32) * ceil_div(p.W / 2, 8 * kSymR) : 0;
@@ -1678,7 +1678,7 @@ void batch_blocks(const Plan2d &p, int blocks[kBatchStages]) {
     blocks[8] = chunked ? ceil_div(p.det, 128) * ceil_div(p.nangles, 8) * 2 : 0;
     blocks[9] = chunked ? 0 : blocks[1];
     blocks[11] = marches(p) ? ceil_div(p.det, 64) * ceil_div(p.nangles, 4) * 2 : 0;
-    blocks[12] = marches(p) ? 0 : blocks[1];
+    blocks[12] = marches(p) ? 0 : ceil_div(p.det, 32) * ceil_div(p.nangles, 8);
 }
 
 bool batch_chunked(const Plan2d &p) {
