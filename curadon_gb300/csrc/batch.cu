@@ -9,9 +9,9 @@
 // calls stream-ordered and capturable in a CUDA graph (an iteration loop is
 // captured once and replayed).
 //
-// The batched forward is the texture-unit ray march (algorithm 1; each
-// problem's volume is copied into its plan's array, then one launch samples
-// all problems through their bindless texture handles), or, selected with
+// The batched forward is the texture-unit ray march (algorithm 1; one launch
+// writes every volume into its plan's array, one samples all problems through
+// their bindless texture handles), or, selected with
 // cg_batch2d_set_forward, the FP32 register march (algorithm 0) or each
 // plan's own default (algorithm 2: the chunked shared-memory forward for
 // problems from 704^2 pixels, one re-layout and one bundle launch over all
@@ -35,7 +35,7 @@ struct cg_batch2d {
     int count = 0;
     int fwd_algo = 1;  // 1 texture unit, 0 registers, 2 each plan's own (chunked / texture)
     std::vector<cg::Plan2d *> plans;
-    std::vector<cg::Prob2d> probs;  // host copy (the texture forward's copies)
+    std::vector<cg::Prob2d> probs;  // host copy of d_probs
     cg::Prob2d *d_probs = nullptr;
     int *d_starts = nullptr;  // kBatchStages stages x (count + 1)
     int totals[cg::kBatchStages] = {};
@@ -157,7 +157,7 @@ int cg_batch2d_create(cg_batch2d **batch, cg_plan2d *const *plans, float *const 
         q.pa = p.pitchA(), q.pb = p.pitchB();
         q.sx = p.sx, q.sy = p.sy, q.ox = p.ox, q.oy = p.oy, q.ds = p.ds;
         if (int rc = ensure_vol_texture(*plans[i])) return rc;
-        q.tex = p.tex_vol, q.arr = p.arr_vol;
+        q.tex = p.tex_vol, q.surf = p.surf_vol;
         q.quadA = p.d_quadA, q.quadB = p.d_quadB;
         q.chunked = batch_chunked(p) ? 1 : 0;
         q.bwd_sym = p.bwd_sym;
@@ -227,12 +227,10 @@ int cg_batch2d_forward(cg_batch2d *batch, void *stream) {
     const Prob2d *probs = all ? batch->d_sorted[0] : batch->d_probs;
     const int *starts = all ? batch->d_sorted_starts[0] : batch->d_starts;
     if (batch->fwd_algo == 1)
-        return launch_batch2d_fwd_tex(probs, batch->probs, batch->active,
-                                      starts + (batch->count + 1), totals[1],
+        return launch_batch2d_fwd_tex(probs, starts, totals, batch->count, 13, 1,
                                       (cudaStream_t)stream);
     if (batch->fwd_algo == 2)
-        return launch_batch2d_fwd_plans(probs, batch->probs, batch->active, starts, totals,
-                                        batch->count, (cudaStream_t)stream);
+        return launch_batch2d_fwd_plans(probs, starts, totals, batch->count, (cudaStream_t)stream);
     return launch_batch2d(probs, starts, totals, batch->count, true, (cudaStream_t)stream);
 }
 

@@ -36,6 +36,7 @@ void free_plan2d(Plan2d *p) {
     if (!p) return;
     if (p->tex_vol) cudaDestroyTextureObject(p->tex_vol);
     if (p->tex_sino) cudaDestroyTextureObject(p->tex_sino);
+    if (p->surf_vol) cudaDestroySurfaceObject(p->surf_vol);
     if (p->arr_vol) cudaFreeArray(p->arr_vol);
     if (p->arr_sino) cudaFreeArray(p->arr_sino);
     void *ptrs[] = {p->d_angles, p->d_DSO,   p->d_DSD,   p->d_src,   p->d_u0,    p->d_du,

@@ -102,6 +102,7 @@ struct Plan2d {
     // texture-unit variants (allocated on first use)
     cudaArray_t arr_vol = nullptr, arr_sino = nullptr;
     cudaTextureObject_t tex_vol = 0, tex_sino = 0;
+    cudaSurfaceObject_t surf_vol = 0;  // arr_vol for writing
 
     // algorithm per operator: forward 0 = registers, 1 = texture unit,
     // 4 = chunked shared-memory slabs; backprojection 0 = registers,
@@ -154,8 +155,8 @@ struct Prob2d {
     float2 *layA, *layB, *sinoP;
     int W, H, det, nangles, pa, pb;
     float sx, sy, ox, oy, ds;
-    cudaTextureObject_t tex;  // the plan's volume texture (texture forward)
-    cudaArray_t arr;          // and its array
+    cudaTextureObject_t tex;   // the plan's volume texture (texture forward)
+    cudaSurfaceObject_t surf;  // and its array for writing
     float4 *quadA, *quadB;    // matched adjoint: the plan's quad accumulators
     int chunked;              // the batched "plans" forward runs the chunked kernel
     int bwd_sym;              // the plan's quarter-turn symmetry (Plan2d::bwd_sym)
@@ -208,8 +209,9 @@ constexpr int kBatch3dStages = 9;
 // texture rays (the others), and the backprojection over the quarter-turn
 // symmetry (problems whose plan has it; stage 3 holds the others).
 // Stages 11 and 12 are the register forward's: bundles, and rays for the
-// problems that have none.
-constexpr int kBatchStages = 13;
+// problems that have none; 13 and 14 fill the texture forward's arrays, of all
+// problems and of those that are not chunked.
+constexpr int kBatchStages = 15;
 // chunked-forward shape the batched "plans" forward compiles
 constexpr int kBatchChunkShape = 484;
 
@@ -322,14 +324,13 @@ int ensure_adj2d_quads(Plan2d &p);
 int launch_batch2d_adjoint(const Prob2d *probs, const int *starts,
                            const int totals[kBatchStages], int count, cudaStream_t s);
 // the "plans" forward: texture rays of the problems that are not chunked
-// (stage 9, after their array copies) and the chunked bundles of the others
-// (stages 7 and 8), the first `active` problems
-int launch_batch2d_fwd_plans(const Prob2d *d_probs, const std::vector<Prob2d> &probs,
-                             int active, const int *starts, const int totals[kBatchStages],
-                             int count, cudaStream_t s);
-int launch_batch2d_fwd_tex_stage(const Prob2d *d_probs, const std::vector<Prob2d> &probs,
-                                 int active, const int *starts, int total, bool only_unchunked,
-                                 cudaStream_t s);
+// (stages 14 and 9) and the chunked bundles of the others (stages 7 and 8)
+int launch_batch2d_fwd_plans(const Prob2d *d_probs, const int *starts,
+                             const int totals[kBatchStages], int count, cudaStream_t s);
+// the texture forward of the stages `fill` (arrays) and `rays` (tiles)
+int launch_batch2d_fwd_tex(const Prob2d *d_probs, const int *starts,
+                           const int totals[kBatchStages], int count, int fill, int rays,
+                           cudaStream_t s);
 int launch_backward2d(const Plan2d &p, float *vol, cudaStream_t s);
 
 int ensure_plan3d_scratch(Plan3d &p, bool fwd, bool bwd);
@@ -353,9 +354,6 @@ int launch_forward2d_cslab(const Plan2d &p, float *sino, cudaStream_t s, int row
 int tex_blocks(const Plan2d &p);
 // The plan's 2D volume texture array and object (allocated once).
 int ensure_vol_texture(Plan2d &p);
-// the first `active` problems of a batch (the work list's blocks [0, total))
-int launch_batch2d_fwd_tex(const Prob2d *d_probs, const std::vector<Prob2d> &probs, int active,
-                           const int *starts, int total, cudaStream_t s);
 int launch_forward2d_tex(Plan2d &p, const float *vol, float *sino, cudaStream_t s);
 int launch_backward2d_tex(Plan2d &p, float *vol, const float *sino, cudaStream_t s);
 // texture forward (tex3D, the reference's trilinear sampling)
@@ -379,6 +377,32 @@ int launch_batch3d_backward(const Prob3d *d_probs, const int *starts,
 int ensure_adj3d_quads(Plan3d &p);
 int launch_batch3d_adjoint(const Prob3d *d_probs, const int *starts,
                            const int totals[kBatch3dStages], int count, cudaStream_t s);
+
+// Launches a kernel that may begin while the stream's previous kernel ends
+// (programmatic dependent launch); cluster_z > 1 makes clusters of that many
+// blocks along z.  Every thread of such a kernel calls wait_previous() before
+// it returns, writes anything or reads what an earlier launch wrote; only the
+// plan's tables, complete since its creation, may be read before.  A dependent
+// launch after a small kernel otherwise costs 2 us of idle GPU (null kernels
+// one after the other 2.06 us, so launched 1.50; a texture forward at 64^2, two
+// launches, 12.0 us a call, so launched 6.3).
+template <class... Params, class... Args>
+int launch_after(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                 unsigned cluster_z, Args... args) {
+    cudaLaunchConfig_t c{};
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = at[1].val.clusterDim.y = 1, at[1].val.clusterDim.z = cluster_z;
+    c.gridDim = grid, c.blockDim = block, c.dynamicSmemBytes = smem, c.stream = s;
+    c.attrs = at, c.numAttrs = cluster_z > 1 ? 2 : 1;
+    CG_TRY_CUDA(cudaLaunchKernelEx(&c, kernel, static_cast<Params>(args)...));
+    return CG_OK;
+}
+#ifdef __CUDACC__
+__device__ __forceinline__ void wait_previous() { cudaGridDependencySynchronize(); }
+#endif
 
 // Reads CURADON_GB300_ALGO ("fwd2d=tex,bwd2d=smem,fwd3d=tex2l,...") over the
 // defaults of a new plan.

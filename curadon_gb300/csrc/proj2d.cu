@@ -1678,6 +1678,8 @@ void batch_blocks(const Plan2d &p, int blocks[kBatchStages]) {
     blocks[8] = chunked ? ceil_div(p.det, 128) * ceil_div(p.nangles, 8) * 2 : 0;
     blocks[9] = chunked ? 0 : blocks[1];
     blocks[11] = marches(p) ? ceil_div(p.det, 64) * ceil_div(p.nangles, 4) * 2 : 0;
+    blocks[13] = ceil_div(p.W, 32) * ceil_div(p.H, 32);
+    blocks[14] = chunked ? 0 : blocks[13];
     blocks[12] = marches(p) ? 0 : ceil_div(p.det, 32) * ceil_div(p.nangles, 8);
 }
 
@@ -1686,11 +1688,9 @@ bool batch_chunked(const Plan2d &p) {
            std::max(p.pitchA(), p.pitchB()) < 32768;
 }
 
-int launch_batch2d_fwd_plans(const Prob2d *d_probs, const std::vector<Prob2d> &probs,
-                             int active, const int *starts, const int totals[kBatchStages],
-                             int count, cudaStream_t s) {
-    int rc = launch_batch2d_fwd_tex_stage(d_probs, probs, active, starts + 9 * (count + 1),
-                                          totals[9], true, s);
+int launch_batch2d_fwd_plans(const Prob2d *d_probs, const int *starts,
+                             const int totals[kBatchStages], int count, cudaStream_t s) {
+    int rc = launch_batch2d_fwd_tex(d_probs, starts, totals, count, 14, 9, s);
     if (rc) return rc;
     if (totals[8] == 0) return CG_OK;
     k_batch_relayout2d_abs<<<totals[7], dim3(32, 8), 0, s>>>(d_probs, starts + 7 * (count + 1),
