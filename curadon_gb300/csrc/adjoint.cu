@@ -97,6 +97,7 @@ __global__ void __launch_bounds__(256)
             const float2 *__restrict__ tsrc, const float2 *__restrict__ tu0,
             const float2 *__restrict__ tdu, int W, int H, int det, int nangles, float sx,
             float sy, int pa, int pb) {
+    wait_previous();
     adj2d_ray<QUAD>(accA, accB, sino, tsrc, tu0, tdu, W, H, det, nangles, sx, sy, pa, pb,
                     blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y);
 }
@@ -115,6 +116,7 @@ __device__ __forceinline__ void fold2d_quad(float *__restrict__ vol, const float
 
 __global__ void k_fold2d_quad(float *__restrict__ vol, const float4 *__restrict__ A,
                               const float4 *__restrict__ B, int W, int H, int pa, int pb) {
+    wait_previous();
     fold2d_quad(vol, A, B, W, H, pa, pb, blockIdx.x * blockDim.x + threadIdx.x,
                 blockIdx.y * blockDim.y + threadIdx.y);
 }
@@ -127,6 +129,7 @@ __global__ void k_fold2d_quad(float *__restrict__ vol, const float4 *__restrict_
 __global__ void __launch_bounds__(256)
     k_batch_adj2d_zero(const Prob2d *__restrict__ probs, const int *__restrict__ start,
                        int count) {
+    wait_previous();
     const int i = batch_problem(start, count, blockIdx.x);
     const Prob2d &q = probs[i];
     const long long na = (long long)q.pa * (q.H + 2 * kPad);
@@ -143,6 +146,7 @@ __global__ void __launch_bounds__(256)
 
 __global__ void __launch_bounds__(256)
     k_batch_adj2d(const Prob2d *__restrict__ probs, const int *__restrict__ start, int count) {
+    wait_previous();
     const int i = batch_problem(start, count, blockIdx.x);
     const Prob2d &q = probs[i];
     const int local = blockIdx.x - start[i];
@@ -154,6 +158,7 @@ __global__ void __launch_bounds__(256)
 
 __global__ void __launch_bounds__(256)
     k_batch_fold2d(const Prob2d *__restrict__ probs, const int *__restrict__ start, int count) {
+    wait_previous();
     const int i = batch_problem(start, count, blockIdx.x);
     const Prob2d &q = probs[i];
     const int local = blockIdx.x - start[i];
@@ -165,6 +170,7 @@ __global__ void __launch_bounds__(256)
 // vol[y][x] += A[y][x].x + A[y][x-1].y + B[x][y].x + B[x][y-1].y (padded).
 __global__ void k_fold2d(float *__restrict__ vol, const float2 *__restrict__ A,
                          const float2 *__restrict__ B, int W, int H, int pa, int pb) {
+    wait_previous();
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y * blockDim.y + threadIdx.y;
     if (x >= W || y >= H) return;
@@ -327,6 +333,7 @@ __global__ void __launch_bounds__(256)
             const float4 *__restrict__ torg, const float4 *__restrict__ tdu,
             const float4 *__restrict__ tdv, const float4 *__restrict__ tsrc, int X, int Y, int Z,
             int U, int V, int P, int utiles, bool exact_t) {
+    wait_previous();
     int iu, iv, view;
     if constexpr (BAND) {
         adj3d_band_cell(blockIdx.x, utiles, P, iu, iv, view);
@@ -342,6 +349,7 @@ __global__ void __launch_bounds__(256)
 // vol[z][y][x] += A[z][y][x].x + A[z][y][x-1].y + B[x][y][z].x + B[x][y][z-1].y
 __global__ void k_fold3d(float *__restrict__ vol, const float2 *__restrict__ A,
                          const float2 *__restrict__ B, int X, int Y, int Z) {
+    wait_previous();
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (long long)X * Y * Z) return;
     const int x = (int)(idx % X);
@@ -373,6 +381,7 @@ __device__ __forceinline__ void fold3d_quad_at(float *__restrict__ vol,
 
 __global__ void k_fold3d_quad(float *__restrict__ vol, const float4 *__restrict__ A,
                               const float4 *__restrict__ B, int X, int Y, int Z) {
+    wait_previous();
     fold3d_quad_at(vol, A, B, X, Y, Z, (long long)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
@@ -384,6 +393,7 @@ __global__ void k_fold3d_quad(float *__restrict__ vol, const float4 *__restrict_
 __global__ void __launch_bounds__(256)
     k_batch_adj3d_zero(const Prob3d *__restrict__ probs, const int *__restrict__ start,
                        int count) {
+    wait_previous();
     const int i = batch_problem(start, count, blockIdx.x);
     const Prob3d &q = probs[i];
     const long long idx = (long long)(blockIdx.x - start[i]) * blockDim.x + threadIdx.x;
@@ -394,6 +404,7 @@ __global__ void __launch_bounds__(256)
 
 __global__ void __launch_bounds__(256)
     k_batch_adj3d(const Prob3d *__restrict__ probs, const int *__restrict__ start, int count) {
+    wait_previous();
     const int i = batch_problem(start, count, blockIdx.x);
     const Prob3d &q = probs[i];
     int iu, iv, view;
@@ -404,6 +415,7 @@ __global__ void __launch_bounds__(256)
 
 __global__ void __launch_bounds__(256)
     k_batch_fold3d(const Prob3d *__restrict__ probs, const int *__restrict__ start, int count) {
+    wait_previous();
     const int i = batch_problem(start, count, blockIdx.x);
     const Prob3d &q = probs[i];
     fold3d_quad_at(q.vol, q.adjA, q.adjB, q.X, q.Y, q.Z,
@@ -426,12 +438,12 @@ int ensure_adj2d_quads(Plan2d &p) {
 int launch_batch2d_adjoint(const Prob2d *probs, const int *starts,
                            const int totals[kBatchStages], int count, cudaStream_t s) {
     const dim3 tile(32, 8);
-    k_batch_adj2d_zero<<<totals[4], 256, 0, s>>>(probs, starts + 4 * (count + 1), count);
-    CG_TRY_CUDA(cudaGetLastError());
-    k_batch_adj2d<<<totals[5], tile, 0, s>>>(probs, starts + 5 * (count + 1), count);
-    CG_TRY_CUDA(cudaGetLastError());
-    k_batch_fold2d<<<totals[6], tile, 0, s>>>(probs, starts + 6 * (count + 1), count);
-    CG_TRY_CUDA(cudaGetLastError());
+    CG_TRY(launch_after(k_batch_adj2d_zero, totals[4], 256, 0, s, 1, probs,
+                        starts + 4 * (count + 1), count));
+    CG_TRY(launch_after(k_batch_adj2d, totals[5], tile, 0, s, 1, probs, starts + 5 * (count + 1),
+                        count));
+    CG_TRY(launch_after(k_batch_fold2d, totals[6], tile, 0, s, 1, probs, starts + 6 * (count + 1),
+                        count));
     return CG_OK;
 }
 
@@ -447,24 +459,20 @@ int launch_adjoint2d(Plan2d &p, float *vol, const float *sino, cudaStream_t s) {
         if (int rc = ensure_adj2d_quads(p)) return rc;
         CG_TRY_CUDA(cudaMemsetAsync(p.d_quadA, 0, na * sizeof(float4), s));
         CG_TRY_CUDA(cudaMemsetAsync(p.d_quadB, 0, nb * sizeof(float4), s));
-        k_adj2d<true><<<grid, block, 0, s>>>(p.d_quadA, p.d_quadB, sino, p.d_src, p.d_u0, p.d_du,
-                                             p.W, p.H, p.det, p.nangles, p.sx, p.sy, p.pitchA(),
-                                             p.pitchB());
-        CG_TRY_CUDA(cudaGetLastError());
-        k_fold2d_quad<<<fgrid, dim3(32, 8), 0, s>>>(vol, p.d_quadA, p.d_quadB, p.W, p.H,
-                                                    p.pitchA(), p.pitchB());
-        CG_TRY_CUDA(cudaGetLastError());
+        CG_TRY(launch_after(k_adj2d<true>, grid, block, 0, s, 1, p.d_quadA, p.d_quadB, sino,
+                            p.d_src, p.d_u0, p.d_du, p.W, p.H, p.det, p.nangles, p.sx, p.sy,
+                            p.pitchA(), p.pitchB()));
+        CG_TRY(launch_after(k_fold2d_quad, fgrid, dim3(32, 8), 0, s, 1, vol, p.d_quadA, p.d_quadB,
+                            p.W, p.H, p.pitchA(), p.pitchB()));
         return CG_OK;
     }
     CG_TRY_CUDA(cudaMemsetAsync(p.d_layA, 0, na * sizeof(float2), s));
     CG_TRY_CUDA(cudaMemsetAsync(p.d_layB, 0, nb * sizeof(float2), s));
-    k_adj2d<false><<<grid, block, 0, s>>>(p.d_layA, p.d_layB, sino, p.d_src, p.d_u0, p.d_du, p.W,
-                                          p.H, p.det, p.nangles, p.sx, p.sy, p.pitchA(),
-                                          p.pitchB());
-    CG_TRY_CUDA(cudaGetLastError());
-    k_fold2d<<<fgrid, dim3(32, 8), 0, s>>>(vol, p.d_layA, p.d_layB, p.W, p.H, p.pitchA(),
-                                           p.pitchB());
-    CG_TRY_CUDA(cudaGetLastError());
+    CG_TRY(launch_after(k_adj2d<false>, grid, block, 0, s, 1, p.d_layA, p.d_layB, sino, p.d_src,
+                        p.d_u0, p.d_du, p.W, p.H, p.det, p.nangles, p.sx, p.sy, p.pitchA(),
+                        p.pitchB()));
+    CG_TRY(launch_after(k_fold2d, fgrid, dim3(32, 8), 0, s, 1, vol, p.d_layA, p.d_layB, p.W, p.H,
+                        p.pitchA(), p.pitchB()));
     return CG_OK;
 }
 
@@ -485,16 +493,16 @@ int launch_batch3d_adjoint(const Prob3d *d_probs, const int *starts,
                            const int totals[kBatch3dStages], int count, cudaStream_t s) {
     const int n1 = count + 1;
     if (totals[6] > 0) {
-        k_batch_adj3d_zero<<<totals[6], 256, 0, s>>>(d_probs, starts + 6 * n1, count);
-        CG_TRY_CUDA(cudaGetLastError());
+        CG_TRY(launch_after(k_batch_adj3d_zero, totals[6], 256, 0, s, 1, d_probs, starts + 6 * n1,
+                            count));
     }
     if (totals[7] > 0) {
-        k_batch_adj3d<<<totals[7], dim3(32, 8), 0, s>>>(d_probs, starts + 7 * n1, count);
-        CG_TRY_CUDA(cudaGetLastError());
+        CG_TRY(launch_after(k_batch_adj3d, totals[7], dim3(32, 8), 0, s, 1, d_probs,
+                            starts + 7 * n1, count));
     }
     if (totals[8] > 0) {
-        k_batch_fold3d<<<totals[8], 256, 0, s>>>(d_probs, starts + 8 * n1, count);
-        CG_TRY_CUDA(cudaGetLastError());
+        CG_TRY(launch_after(k_batch_fold3d, totals[8], 256, 0, s, 1, d_probs, starts + 8 * n1,
+                            count));
     }
     return CG_OK;
 }
@@ -522,23 +530,21 @@ int launch_adjoint3d(Plan3d &p, float *vol, const float *sino, cudaStream_t s) {
                                       : k_adj3d<true, false, true, true>)
                   : p.adj_merge ? (band ? k_adj3d<true, true, true> : k_adj3d<true, false, true>)
                                 : (band ? k_adj3d<true, true> : k_adj3d<true, false>);
-        kq<<<grid, dim3(32, 8), 0, s>>>(p.d_quadA, p.d_quadB, sino, p.d_forg, p.d_fdu, p.d_fdv,
-                                        p.d_fsrc, p.X, p.Y, p.Z, p.U, p.V, p.nangles, utiles,
-                                        p.exact_t);
-        CG_TRY_CUDA(cudaGetLastError());
-        k_fold3d_quad<<<ceil_div(n, 256), 256, 0, s>>>(vol, p.d_quadA, p.d_quadB, p.X, p.Y, p.Z);
-        CG_TRY_CUDA(cudaGetLastError());
+        CG_TRY(launch_after(kq, grid, dim3(32, 8), 0, s, 1, p.d_quadA, p.d_quadB, sino, p.d_forg,
+                            p.d_fdu, p.d_fdv, p.d_fsrc, p.X, p.Y, p.Z, p.U, p.V, p.nangles, utiles,
+                            p.exact_t));
+        CG_TRY(launch_after(k_fold3d_quad, ceil_div(n, 256), 256, 0, s, 1, vol, p.d_quadA,
+                            p.d_quadB, p.X, p.Y, p.Z));
         return CG_OK;
     }
     CG_TRY_CUDA(cudaMemsetAsync(p.d_volA, 0, p.volA_elems * sizeof(float2), s));
     CG_TRY_CUDA(cudaMemsetAsync(p.d_volB, 0, p.volB_elems * sizeof(float2), s));
     auto kp = band ? k_adj3d<false, true> : k_adj3d<false, false>;
-    kp<<<grid, dim3(32, 8), 0, s>>>(p.d_volA, p.d_volB, sino, p.d_forg, p.d_fdu, p.d_fdv,
-                                    p.d_fsrc, p.X, p.Y, p.Z, p.U, p.V, p.nangles, utiles,
-                                    p.exact_t);
-    CG_TRY_CUDA(cudaGetLastError());
-    k_fold3d<<<ceil_div(n, 256), 256, 0, s>>>(vol, p.d_volA, p.d_volB, p.X, p.Y, p.Z);
-    CG_TRY_CUDA(cudaGetLastError());
+    CG_TRY(launch_after(kp, grid, dim3(32, 8), 0, s, 1, p.d_volA, p.d_volB, sino, p.d_forg,
+                        p.d_fdu, p.d_fdv, p.d_fsrc, p.X, p.Y, p.Z, p.U, p.V, p.nangles, utiles,
+                        p.exact_t));
+    CG_TRY(launch_after(k_fold3d, ceil_div(n, 256), 256, 0, s, 1, vol, p.d_volA, p.d_volB, p.X,
+                        p.Y, p.Z));
     return CG_OK;
 }
 

@@ -30,6 +30,12 @@ void clear_error();
         }                                                                                     \
     } while (0)
 
+// Returns the status of a call of ours unless it is CG_OK.
+#define CG_TRY(expr)                                                                          \
+    do {                                                                                      \
+        if (int cg_rc_ = (expr)) return cg_rc_;                                               \
+    } while (0)
+
 #define CG_REQUIRE(cond, msg)                                                                 \
     do {                                                                                      \
         if (!(cond)) return ::cg::set_error(CG_ERR_INVALID, (msg));                           \
@@ -385,10 +391,11 @@ int launch_batch3d_adjoint(const Prob3d *d_probs, const int *starts,
 // plan's tables, complete since its creation, may be read before.  A dependent
 // launch after a small kernel otherwise costs 2 us of idle GPU (null kernels
 // one after the other 2.06 us, so launched 1.50; a texture forward at 64^2, two
-// launches, 12.0 us a call, so launched 6.3).
+// launches, 12.0 us a call, so launched 6.3; a 512^2 x 512 backprojection 72 us,
+// 67; filtered backprojection at 1024^2 445 us, 435).
 template <class... Params, class... Args>
 int launch_after(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
-                 unsigned cluster_z, Args... args) {
+                 unsigned cluster_z, const Args &...args) {
     cudaLaunchConfig_t c{};
     cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -397,7 +404,7 @@ int launch_after(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, 
     at[1].val.clusterDim.x = at[1].val.clusterDim.y = 1, at[1].val.clusterDim.z = cluster_z;
     c.gridDim = grid, c.blockDim = block, c.dynamicSmemBytes = smem, c.stream = s;
     c.attrs = at, c.numAttrs = cluster_z > 1 ? 2 : 1;
-    CG_TRY_CUDA(cudaLaunchKernelEx(&c, kernel, static_cast<Params>(args)...));
+    CG_TRY_CUDA(cudaLaunchKernelEx(&c, kernel, args...));
     return CG_OK;
 }
 #ifdef __CUDACC__

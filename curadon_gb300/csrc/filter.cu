@@ -55,6 +55,7 @@ __global__ void __launch_bounds__(kFiltThreads)
     k_filter_rows(const float *__restrict__ in, float *__restrict__ out,
                   const float *__restrict__ h, const float *__restrict__ pre, int nrows, int N,
                   float scale, bool skip_ramp) {
+    wait_previous();
     if (skip_ramp && ramp_taps(h, N)) return;
     extern __shared__ float smem[];
     float *sh = smem;            // N
@@ -113,6 +114,7 @@ __global__ void __launch_bounds__(kFiltThreads)
     k_filter_rows_pk(const float *__restrict__ in, float *__restrict__ out,
                      const float *__restrict__ h, const float *__restrict__ pre, int nrows, int N,
                      float scale, bool skip_ramp) {
+    wait_previous();
     if (skip_ramp && ramp_taps(h, N)) return;
     static_assert(RB % 2 == 0, "row pairs");
     extern __shared__ float2 smem2[];
@@ -172,9 +174,8 @@ int launch_rb_pk(const float *in, float *out, const float *h, const float *pre, 
     const size_t smem = sizeof(float2) * (size_t)N * (RB / 2 + 1);
     if (int rc = ensure_smem_attr((const void *)k_filter_rows_pk<RB>, (int)smem)) return rc;
     dim3 grid(ceil_div(N, kFiltThreads * kFiltOut), ceil_div(nrows, RB));
-    k_filter_rows_pk<RB><<<grid, kFiltThreads, smem, s>>>(in, out, h, pre, nrows, N, scale,
-                                                          skip_ramp);
-    CG_TRY_CUDA(cudaGetLastError());
+    CG_TRY(launch_after(k_filter_rows_pk<RB>, grid, kFiltThreads, smem, s, 1, in, out, h, pre,
+                        nrows, N, scale, skip_ramp));
     return CG_OK;
 }
 
@@ -184,9 +185,8 @@ int launch_rb(const float *in, float *out, const float *h, const float *pre, int
     const size_t smem = sizeof(float) * (size_t)N * (RB + 1);
     if (int rc = ensure_smem_attr((const void *)k_filter_rows<RB>, (int)smem)) return rc;
     dim3 grid(ceil_div(N, kFiltThreads * kFiltOut), ceil_div(nrows, RB));
-    k_filter_rows<RB><<<grid, kFiltThreads, smem, s>>>(in, out, h, pre, nrows, N, scale,
-                                                       skip_ramp);
-    CG_TRY_CUDA(cudaGetLastError());
+    CG_TRY(launch_after(k_filter_rows<RB>, grid, kFiltThreads, smem, s, 1, in, out, h, pre, nrows,
+                        N, scale, skip_ramp));
     return CG_OK;
 }
 
@@ -329,6 +329,7 @@ __global__ void __launch_bounds__(RowFft<C>::T *RowFft<C>::G)
     k_filter_fft(const float *__restrict__ in, float *__restrict__ out,
                  const float *__restrict__ h, const float *__restrict__ pre, int nrows, int N,
                  float scale) {
+    wait_previous();
     using F = RowFft<C>;
     constexpr int T = F::T, G = F::G, M = 2 * C;
     extern __shared__ float2 fsm[];
@@ -510,8 +511,8 @@ int launch_fft(const float *in, float *out, const float *h, const float *pre, in
                                                               F::T * F::G, F::smem));
     const int slots = std::max(1, resident * sm_count()), groups = ceil_div(nrows, F::G);
     const int blocks = ceil_div(groups, ceil_div(groups, slots));
-    k_filter_fft<C><<<blocks, F::T * F::G, F::smem, s>>>(in, out, h, pre, nrows, N, scale);
-    CG_TRY_CUDA(cudaGetLastError());
+    CG_TRY(launch_after(k_filter_fft<C>, blocks, F::T * F::G, F::smem, s, 1, in, out, h, pre,
+                        nrows, N, scale));
     return CG_OK;
 }
 

@@ -119,6 +119,7 @@ template <bool ABS>
 __global__ void __launch_bounds__(256)
     k_relayout2d(const float *__restrict__ vol, int W, int H, float2 *__restrict__ A,
                  float2 *__restrict__ B, int pa, int pb) {
+    wait_previous();
     relayout2d_tile<ABS>(vol, W, H, A, B, pa, pb, blockIdx.x, blockIdx.y);
 }
 
@@ -142,6 +143,7 @@ __device__ __forceinline__ void relayout_sino2d_elem(const float *__restrict__ s
 template <bool ABS>
 __global__ void k_relayout_sino2d(const float *__restrict__ sino, int det, int nangles,
                                   float2 *__restrict__ S) {
+    wait_previous();
     relayout_sino2d_elem<ABS>(sino, det, nangles, S,
                               (long long)blockIdx.x * blockDim.x + threadIdx.x);
 }
@@ -229,6 +231,7 @@ __global__ void __launch_bounds__(256)
             float *__restrict__ sino, const float2 *__restrict__ tsrc,
             const float2 *__restrict__ tu0, const float2 *__restrict__ tdu, int W, int H,
             int det, int nangles, float sx, float sy, int pa, int pb) {
+    wait_previous();
     fwd2d_ray(layA, layB, sino, tsrc, tu0, tdu, W, H, det, nangles, sx, sy, pa, pb,
               blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y);
 }
@@ -712,6 +715,7 @@ __global__ void __launch_bounds__(T * VS, MB)
                   float *__restrict__ sino, const float2 *__restrict__ tsrc,
                   const float2 *__restrict__ tu0, const float2 *__restrict__ tdu, int W, int H,
                   int det, int nangles, float sx, float sy, int pa, int pb) {
+    wait_previous();
     cslab_bundle<K, S, T, PK, REUSE, VS, NG, MB, MAP, ABS, TMA>(
         layA, layB, sino, tsrc, tu0, tdu, W, H, det, nangles, sx, sy, pa, pb, blockIdx.x,
         blockIdx.y, blockIdx.z);
@@ -744,6 +748,7 @@ __global__ void __launch_bounds__(128, 5)
                   float *__restrict__ sino, const float2 *__restrict__ tsrc,
                   const float2 *__restrict__ tu0, const float2 *__restrict__ tdu, int W, int H,
                   int det, int nangles, float sx, float sy, int pa, int pb) {
+    wait_previous();
     march_bundle(layA, layB, sino, tsrc, tu0, tdu, W, H, det, nangles, sx, sy, pa, pb, blockIdx.x,
                  blockIdx.y, blockIdx.z);
 }
@@ -786,10 +791,9 @@ int launch_forward2d_cslab(const Plan2d &p, float *sino, cudaStream_t s, int row
         const size_t smem = cslab_smem(stride);
         if (int rc = ensure_smem_attr((const void *)kernel, (int)smem)) return rc;
         dim3 grid(ceil_div(p.det, cells), ceil_div(p.nangles, views), 2);
-        kernel<<<grid, cells * 2, smem, s>>>(p.d_layA, p.d_layB, sino, p.d_src, p.d_u0, p.d_du,
-                                             p.W, p.H, p.det, p.nangles, p.sx, p.sy, p.pitchA(),
-                                             p.pitchB());
-        CG_TRY_CUDA(cudaGetLastError());
+        CG_TRY(launch_after(kernel, grid, cells * 2, smem, s, 1, p.d_layA, p.d_layB, sino, p.d_src,
+                            p.d_u0, p.d_du, p.W, p.H, p.det, p.nangles, p.sx, p.sy, p.pitchA(),
+                            p.pitchB()));
         return CG_OK;
     };
     // the default (484) and the autotuner's other candidates (474: the same
@@ -824,6 +828,7 @@ __global__ void __launch_bounds__(256)
     k_bwd2d(float *__restrict__ vol, const float2 *__restrict__ S,
             const float4 *__restrict__ meta, int W, int H, int det, int nangles, float sx,
             float sy, float ox, float oy, float ds) {
+    wait_previous();
     __shared__ float4 smeta[kBwdViews];
     const int tid = threadIdx.y * blockDim.x + threadIdx.x;
     const int x = blockIdx.x * 32 + threadIdx.x;
@@ -1453,6 +1458,7 @@ __global__ void __launch_bounds__(256, MINB)
     k_bwd2d_sym(float *__restrict__ vol, const float2 *__restrict__ S,
                 const float4 *__restrict__ proj, int W, int det, int nangles, float sx, float ox,
                 float ds, int dir) {
+    wait_previous();
     bwd2d_sym_tile<kSymR, kSymNV, kSymWin>(vol, S, proj, W, det, nangles, sx, ox, ds, dir,
                                            blockIdx.x, blockIdx.y);
 }
@@ -1464,6 +1470,7 @@ __global__ void __launch_bounds__(256, MINB)
     k_bwd2d_smem(float *__restrict__ vol, const float2 *__restrict__ S,
                  const float4 *__restrict__ proj, int W, int H, int det, int nangles, float sx,
                  float sy, float ox, float oy, float ds, int per) {
+    wait_previous();
     bwd2d_smem_tile<PK, MAGIC, VU, CPA, ABS, MAPQ, BULK, R>(vol, S, proj, W, H, det, nangles,
                                                             sx, sy, ox, oy, ds, blockIdx.x,
                                                             blockIdx.y, per);
@@ -1480,6 +1487,7 @@ __global__ void __launch_bounds__(32 * G)
     k_bwd2d_direct(float *__restrict__ vol, const float *__restrict__ sino,
                    const float4 *__restrict__ proj, int W, int H, int det, int nangles, float sx,
                    float sy, float ox, float oy, float ds, int per) {
+    wait_previous();
     __shared__ float4 sA[G][32], sB[G][32];
     __shared__ float part[G][64];
     const int lane = threadIdx.x, group = threadIdx.y, groups = blockDim.y;
@@ -1543,6 +1551,7 @@ __global__ void __launch_bounds__(256, MINB)
     k_bwd2d_cluster(float *__restrict__ vol, const float2 *__restrict__ S,
                     const float4 *__restrict__ proj, int W, int H, int det, int nangles, float sx,
                     float sy, float ox, float oy, float ds, int per) {
+    wait_previous();
     bwd2d_smem_tile<true, true, 4, true, true, true, true, kSmRows, true>(
         vol, S, proj, W, H, det, nangles, sx, sy, ox, oy, ds, blockIdx.x, blockIdx.y, per,
         blockIdx.z);
@@ -1562,6 +1571,7 @@ namespace {
 
 __global__ void __launch_bounds__(256)
     k_batch_relayout2d(const Prob2d *__restrict__ probs, const int *__restrict__ start, int count) {
+    wait_previous();
     const int i = batch_problem(start, count, blockIdx.x);
     const Prob2d &q = probs[i];
     const int local = blockIdx.x - start[i];
@@ -1572,6 +1582,7 @@ __global__ void __launch_bounds__(256)
 __global__ void __launch_bounds__(256)
     k_batch_relayout2d_abs(const Prob2d *__restrict__ probs, const int *__restrict__ start,
                            int count) {
+    wait_previous();
     const int i = batch_problem(start, count, blockIdx.x);
     const Prob2d &q = probs[i];
     const int local = blockIdx.x - start[i];
@@ -1584,6 +1595,7 @@ __global__ void __launch_bounds__(256)
 __global__ void __launch_bounds__(256, 3)
     k_batch_fwd2d_cslab(const Prob2d *__restrict__ probs, const int *__restrict__ start,
                         int count) {
+    wait_previous();
     const int i = batch_problem(start, count, blockIdx.x);
     const Prob2d &q = probs[i];
     const int local = blockIdx.x - start[i];
@@ -1598,6 +1610,7 @@ __global__ void __launch_bounds__(256, 3)
 __global__ void __launch_bounds__(128, 5)
     k_batch_fwd2d_march(const Prob2d *__restrict__ probs, const int *__restrict__ start,
                         int count) {
+    wait_previous();
     const int i = batch_problem(start, count, blockIdx.x);
     const Prob2d &q = probs[i];
     const int local = blockIdx.x - start[i];
@@ -1608,6 +1621,7 @@ __global__ void __launch_bounds__(128, 5)
 
 __global__ void __launch_bounds__(256)
     k_batch_fwd2d(const Prob2d *__restrict__ probs, const int *__restrict__ start, int count) {
+    wait_previous();
     const int i = batch_problem(start, count, blockIdx.x);
     const Prob2d &q = probs[i];
     const int local = blockIdx.x - start[i];
@@ -1619,6 +1633,7 @@ __global__ void __launch_bounds__(256)
 __global__ void __launch_bounds__(256)
     k_batch_relayout_sino2d(const Prob2d *__restrict__ probs, const int *__restrict__ start,
                             int count) {
+    wait_previous();
     const int i = batch_problem(start, count, blockIdx.x);
     const Prob2d &q = probs[i];
     const long long idx = (long long)(blockIdx.x - start[i]) * blockDim.x + threadIdx.x;
@@ -1631,6 +1646,7 @@ __global__ void __launch_bounds__(256)
 // bit.
 __global__ void __launch_bounds__(256, 4)
     k_batch_bwd2d(const Prob2d *__restrict__ probs, const int *__restrict__ start, int count) {
+    wait_previous();
     const int i = batch_problem(start, count, blockIdx.x);
     const Prob2d &q = probs[i];
     const int local = blockIdx.x - start[i];
@@ -1646,6 +1662,7 @@ __global__ void __launch_bounds__(256, 4)
 __global__ void __launch_bounds__(256, 4)
     k_batch_bwd2d_sym(const Prob2d *__restrict__ probs, const int *__restrict__ start,
                       int count) {
+    wait_previous();
     const int i = batch_problem(start, count, blockIdx.x);
     const Prob2d &q = probs[i];
     const int local = blockIdx.x - start[i];
@@ -1693,13 +1710,12 @@ int launch_batch2d_fwd_plans(const Prob2d *d_probs, const int *starts,
     int rc = launch_batch2d_fwd_tex(d_probs, starts, totals, count, 14, 9, s);
     if (rc) return rc;
     if (totals[8] == 0) return CG_OK;
-    k_batch_relayout2d_abs<<<totals[7], dim3(32, 8), 0, s>>>(d_probs, starts + 7 * (count + 1),
-                                                             count);
-    CG_TRY_CUDA(cudaGetLastError());
+    CG_TRY(launch_after(k_batch_relayout2d_abs, totals[7], dim3(32, 8), 0, s, 1, d_probs,
+                        starts + 7 * (count + 1), count));
     const size_t smem = cslab_smem(kCsCols);
     if ((rc = ensure_smem_attr((const void *)k_batch_fwd2d_cslab, (int)smem))) return rc;
-    k_batch_fwd2d_cslab<<<totals[8], 256, smem, s>>>(d_probs, starts + 8 * (count + 1), count);
-    CG_TRY_CUDA(cudaGetLastError());
+    CG_TRY(launch_after(k_batch_fwd2d_cslab, totals[8], 256, smem, s, 1, d_probs,
+                        starts + 8 * (count + 1), count));
     return CG_OK;
 }
 
@@ -1707,28 +1723,26 @@ int launch_batch2d(const Prob2d *probs, const int *starts, const int totals[kBat
                    int count, bool forward, cudaStream_t s) {
     const dim3 tile(32, 8);
     if (forward) {
-        k_batch_relayout2d<<<totals[0], tile, 0, s>>>(probs, starts, count);
-        CG_TRY_CUDA(cudaGetLastError());
+        CG_TRY(launch_after(k_batch_relayout2d, totals[0], tile, 0, s, 1, probs, starts, count));
         if (totals[11] > 0) {
             const size_t smem = cslab_smem(kCsSmallCols);
             if (int rc = ensure_smem_attr((const void *)k_batch_fwd2d_march, (int)smem)) return rc;
-            k_batch_fwd2d_march<<<totals[11], 128, smem, s>>>(probs, starts + 11 * (count + 1),
-                                                              count);
-            CG_TRY_CUDA(cudaGetLastError());
+            CG_TRY(launch_after(k_batch_fwd2d_march, totals[11], 128, smem, s, 1, probs,
+                                starts + 11 * (count + 1), count));
         }
         if (totals[12] > 0)
-            k_batch_fwd2d<<<totals[12], tile, 0, s>>>(probs, starts + 12 * (count + 1), count);
+            CG_TRY(launch_after(k_batch_fwd2d, totals[12], tile, 0, s, 1, probs,
+                                starts + 12 * (count + 1), count));
     } else {
-        k_batch_relayout_sino2d<<<totals[2], 256, 0, s>>>(probs, starts + 2 * (count + 1), count);
-        CG_TRY_CUDA(cudaGetLastError());
+        CG_TRY(launch_after(k_batch_relayout_sino2d, totals[2], 256, 0, s, 1, probs,
+                            starts + 2 * (count + 1), count));
         if (totals[3] > 0)
-            k_batch_bwd2d<<<totals[3], tile, 0, s>>>(probs, starts + 3 * (count + 1), count);
-        CG_TRY_CUDA(cudaGetLastError());
+            CG_TRY(launch_after(k_batch_bwd2d, totals[3], tile, 0, s, 1, probs,
+                                starts + 3 * (count + 1), count));
         if (totals[10] > 0)
-            k_batch_bwd2d_sym<<<totals[10], tile, 0, s>>>(probs, starts + 10 * (count + 1),
-                                                          count);
+            CG_TRY(launch_after(k_batch_bwd2d_sym, totals[10], tile, 0, s, 1, probs,
+                                starts + 10 * (count + 1), count));
     }
-    CG_TRY_CUDA(cudaGetLastError());
     return CG_OK;
 }
 
@@ -1749,9 +1763,8 @@ int launch_relayout2d(const Plan2d &p, const float *vol, cudaStream_t s) {
     // the chunked forward's absolute-position shapes read the ABS form
     const bool abs_form = (p.algo_fwd == 4 || p.algo_fwd == 5) && cslab_abs(p.fwd_chunk_rows);
     auto kernel = abs_form ? k_relayout2d<true> : k_relayout2d<false>;
-    kernel<<<grid, dim3(32, 8), 0, s>>>(vol, p.W, p.H, p.d_layA, p.d_layB, p.pitchA(),
-                                        p.pitchB());
-    CG_TRY_CUDA(cudaGetLastError());
+    CG_TRY(launch_after(kernel, grid, dim3(32, 8), 0, s, 1, vol, p.W, p.H, p.d_layA, p.d_layB,
+                        p.pitchA(), p.pitchB()));
     return CG_OK;
 }
 
@@ -1760,18 +1773,16 @@ int launch_forward2d(const Plan2d &p, float *sino, cudaStream_t s) {
         const size_t smem = cslab_smem(kCsSmallCols);
         if (int rc = ensure_smem_attr((const void *)k_fwd2d_march, (int)smem)) return rc;
         const dim3 grid(ceil_div(p.det, 64), ceil_div(p.nangles, 4), 2);
-        k_fwd2d_march<<<grid, 128, smem, s>>>(p.d_layA, p.d_layB, sino, p.d_src, p.d_u0, p.d_du,
-                                              p.W, p.H, p.det, p.nangles, p.sx, p.sy, p.pitchA(),
-                                              p.pitchB());
-        CG_TRY_CUDA(cudaGetLastError());
+        CG_TRY(launch_after(k_fwd2d_march, grid, 128, smem, s, 1, p.d_layA, p.d_layB, sino,
+                            p.d_src, p.d_u0, p.d_du, p.W, p.H, p.det, p.nangles, p.sx, p.sy,
+                            p.pitchA(), p.pitchB()));
         return CG_OK;
     }
     dim3 block(p.fwd_bx, p.fwd_by);
     dim3 grid(ceil_div(p.det, p.fwd_bx), ceil_div(p.nangles, p.fwd_by));
     if (grid.y > 65535) return set_error(CG_ERR_INVALID, "too many views for one launch");
-    k_fwd2d<<<grid, block, 0, s>>>(p.d_layA, p.d_layB, sino, p.d_src, p.d_u0, p.d_du, p.W, p.H,
-                                   p.det, p.nangles, p.sx, p.sy, p.pitchA(), p.pitchB());
-    CG_TRY_CUDA(cudaGetLastError());
+    CG_TRY(launch_after(k_fwd2d, grid, block, 0, s, 1, p.d_layA, p.d_layB, sino, p.d_src, p.d_u0,
+                        p.d_du, p.W, p.H, p.det, p.nangles, p.sx, p.sy, p.pitchA(), p.pitchB()));
     return CG_OK;
 }
 
@@ -1780,8 +1791,8 @@ int launch_relayout_sino2d(const Plan2d &p, const float *sino, cudaStream_t s) {
     // the staged backprojector's absolute-position shapes read the ABS form
     const bool abs_form = (p.algo_bwd == 2 || p.algo_bwd == 3) && bwd_abs(p.bwd_min_blocks);
     auto kernel = abs_form ? k_relayout_sino2d<true> : k_relayout_sino2d<false>;
-    kernel<<<ceil_div(n, 256), 256, 0, s>>>(sino, p.det, p.nangles, p.d_sinoP);
-    CG_TRY_CUDA(cudaGetLastError());
+    CG_TRY(launch_after(kernel, ceil_div(n, 256), 256, 0, s, 1, sino, p.det, p.nangles,
+                        p.d_sinoP));
     return CG_OK;
 }
 
@@ -1846,28 +1857,19 @@ int bwd_group_views(const Plan2d &p) {
 
 int launch_backward2d_smem(const Plan2d &p, float *vol, const float *sino, cudaStream_t s) {
     const int per = bwd_group_views(p), groups = ceil_div(p.nangles, per);
-    auto go = [&](auto kernel, dim3 grid, dim3 block, unsigned cluster, auto... args) -> int {
-        cudaLaunchConfig_t c{};
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = at[0].val.clusterDim.y = 1, at[0].val.clusterDim.z = cluster;
-        c.gridDim = grid, c.blockDim = block, c.stream = s, c.attrs = at;
-        c.numAttrs = cluster > 1 ? 1 : 0;
-        CG_TRY_CUDA(cudaLaunchKernelEx(&c, kernel, vol, args...));
-        return CG_OK;
-    };
     const bool standard = p.bwd_min_blocks == 68;
     if (standard && bwd_direct(p))
-        return go(groups > 4 ? k_bwd2d_direct<kDirectGroups> : k_bwd2d_direct<4>,
-                  dim3(ceil_div(p.W, 8), ceil_div(p.H, 8)), dim3(32, groups), 1, sino, (const float4 *)p.d_bproj, p.W, p.H, p.det, p.nangles, p.sx, p.sy, p.ox,
-                  p.oy, p.ds, per);
+        return launch_after(groups > 4 ? k_bwd2d_direct<kDirectGroups> : k_bwd2d_direct<4>,
+                            dim3(ceil_div(p.W, 8), ceil_div(p.H, 8)), dim3(32, groups), 0, s, 1,
+                            vol, sino, p.d_bproj, p.W, p.H, p.det, p.nangles, p.sx, p.sy, p.ox,
+                            p.oy, p.ds, per);
     if (int rc = launch_relayout_sino2d(p, sino, s)) return rc;
     if (p.bwd_sym != 0) {
         // the first quadrant's tiles, each with its three turned copies
         const int half = p.W / 2;
-        return go(k_bwd2d_sym<4>, dim3(ceil_div(half, 32), ceil_div(half, 8 * kSymR)), dim3(32, 8), 1,
-                  (const float2 *)p.d_sinoP, (const float4 *)p.d_bproj, p.W, p.det, p.nangles, p.sx,
-                  p.ox, p.ds, p.bwd_sym);
+        return launch_after(k_bwd2d_sym<4>, dim3(ceil_div(half, 32), ceil_div(half, 8 * kSymR)),
+                            dim3(32, 8), 0, s, 1, vol, p.d_sinoP, p.d_bproj, p.W, p.det, p.nangles,
+                            p.sx, p.ox, p.ds, p.bwd_sym);
     }
     // tiles of 32 x 64 pixels; an image whose tiles would not give every SM
     // two blocks takes 32 x 16-pixel tiles (two pixels per thread) instead,
@@ -1876,9 +1878,10 @@ int launch_backward2d_smem(const Plan2d &p, float *vol, const float *sino, cudaS
     const bool small = !cluster && (long long)ceil_div(p.W, 32) * ceil_div(p.H, 8 * kSmRows) < 2LL * sm_count();
     auto tile = [&](auto kernel) {
         const unsigned z = cluster ? groups : 1;
-        return go(kernel, dim3(ceil_div(p.W, 32), ceil_div(p.H, 8 * (small ? 2 : kSmRows)), z),
-                  dim3(32, 8), z, (const float2 *)p.d_sinoP, (const float4 *)p.d_bproj, p.W, p.H,
-                  p.det, p.nangles, p.sx, p.sy, p.ox, p.oy, p.ds, per);
+        return launch_after(kernel,
+                            dim3(ceil_div(p.W, 32), ceil_div(p.H, 8 * (small ? 2 : kSmRows)), z),
+                            dim3(32, 8), 0, s, z, vol, p.d_sinoP, p.d_bproj, p.W, p.H, p.det,
+                            p.nangles, p.sx, p.sy, p.ox, p.oy, p.ds, per);
     };
     if (cluster) return tile(k_bwd2d_cluster<4>);
     // the default (68) and the autotuner's other candidates (48: the same
@@ -1899,9 +1902,8 @@ int launch_backward2d_smem(const Plan2d &p, float *vol, const float *sino, cudaS
 
 int launch_backward2d(const Plan2d &p, float *vol, cudaStream_t s) {
     dim3 grid(ceil_div(p.W, 32), ceil_div(p.H, 32));
-    k_bwd2d<<<grid, dim3(32, 8), 0, s>>>(vol, p.d_sinoP, p.d_bmeta, p.W, p.H, p.det, p.nangles,
-                                         p.sx, p.sy, p.ox, p.oy, p.ds);
-    CG_TRY_CUDA(cudaGetLastError());
+    CG_TRY(launch_after(k_bwd2d, grid, dim3(32, 8), 0, s, 1, vol, p.d_sinoP, p.d_bmeta, p.W, p.H,
+                        p.det, p.nangles, p.sx, p.sy, p.ox, p.oy, p.ds));
     return CG_OK;
 }
 

@@ -27,6 +27,7 @@ constexpr int kQP = 2 * kP3 + 1;  // quad copies: kP3 zero planes below, kP3 + 1
 
 __global__ void k_relayout3d_A(const float *__restrict__ vol, int X, int Y, int Z,
                                float2 *__restrict__ A) {
+    wait_previous();
     const int PX = X + 2 * kP3, PY = Y + 2 * kP3, PZ = Z + 2 * kP3;
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (long long)PX * PY * PZ) return;
@@ -46,6 +47,7 @@ __global__ void k_relayout3d_A(const float *__restrict__ vol, int X, int Y, int 
 // x <-> z transpose of one y plane, 32 x 32 tiles through shared memory.
 __global__ void __launch_bounds__(256)
     k_relayout3d_B(const float *__restrict__ vol, int X, int Y, int Z, float2 *__restrict__ B) {
+    wait_previous();
     __shared__ float tile[33][33];  // [z][x]
     const int PY = Y + 2 * kP3, PZ = Z + 2 * kP3, PX = X + 2 * kP3;
     const int x0 = blockIdx.x * 32 - kP3, z0 = blockIdx.y * 32 - kP3;
@@ -99,6 +101,7 @@ __device__ __forceinline__ void relayout3d_qa_at(const float *__restrict__ vol, 
 
 __global__ void k_relayout3d_qa(const float *__restrict__ vol, int X, int Y, int Z,
                                 float4 *__restrict__ QA) {
+    wait_previous();
     relayout3d_qa_at(vol, X, Y, Z, QA, (long long)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
@@ -133,12 +136,14 @@ __device__ __forceinline__ void relayout3d_qb_tile(const float *__restrict__ vol
 
 __global__ void __launch_bounds__(256)
     k_relayout3d_qb(const float *__restrict__ vol, int X, int Y, int Z, float4 *__restrict__ QB) {
+    wait_previous();
     relayout3d_qb_tile(vol, X, Y, Z, QB, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
 
 __global__ void k_relayout_sino3d(const float *__restrict__ sino, int U, int V, int nangles,
                                   float2 *__restrict__ S) {
+    wait_previous();
     const int PU = U + 2 * kP3, PV = V + 2 * kP3;
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (long long)PU * PV * nangles) return;
@@ -179,6 +184,7 @@ __device__ __forceinline__ void relayout_sino3d_quad_at(const float *__restrict_
 
 __global__ void k_relayout_sino3d_quad(const float *__restrict__ sino, int U, int V, int nangles,
                                        float4 *__restrict__ S) {
+    wait_previous();
     relayout_sino3d_quad_at(sino, U, V, nangles, S, (long long)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
@@ -208,6 +214,7 @@ __device__ __forceinline__ void relayout_sino3d_qd_at(const float *__restrict__ 
 
 __global__ void k_relayout_sino3d_qd(const float *__restrict__ sino, int U, int V, int nangles,
                                      float4 *__restrict__ S) {
+    wait_previous();
     relayout_sino3d_qd_at(sino, U, V, nangles, S, (long long)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
@@ -222,6 +229,7 @@ __global__ void __launch_bounds__(256)
             const float4 *__restrict__ torg, const float4 *__restrict__ tdu,
             const float4 *__restrict__ tdv, const float4 *__restrict__ tsrc, int X, int Y, int Z,
             int U, int V, bool exact_t) {
+    wait_previous();
     const int iu = blockIdx.x * blockDim.x + threadIdx.x;
     const int iv = blockIdx.y * blockDim.y + threadIdx.y;
     const int view = blockIdx.z;
@@ -478,6 +486,7 @@ __global__ void __launch_bounds__(256)
                  const float4 *__restrict__ tdu, const float4 *__restrict__ tdv,
                  const float4 *__restrict__ tsrc, int X, int Y, int Z, int U, int V, int P,
                  int utiles, cudaTextureObject_t tex, int tex_warps, bool exact_t) {
+    wait_previous();
     fwd3d_quad_block<UNR>(QA, QB, sino, torg, tdu, tdv, tsrc, X, Y, Z, U, V, P, utiles, tex,
                           tex_warps, exact_t, blockIdx.x);
 }
@@ -650,6 +659,7 @@ __global__ void __launch_bounds__(256)
             const float4 *__restrict__ tdy, const float4 *__restrict__ tdz, float srcx,
             float srcy, float srcz, float zplane, float hu, float hv, int X, int Y, int Z, int U,
             int V, int nangles, int tiles_x, int tiles_y, int tiles_z) {
+    wait_previous();
     bwd3d_block<PK, MAGIC, QS>(vol, Sv, torg, tdx, tdy, tdz, srcx, srcy, srcz, zplane, hu, hv, X,
                                Y, Z, U, V, nangles, tiles_x, tiles_y, tiles_z, blockIdx.x);
 }
@@ -761,6 +771,7 @@ __global__ void __launch_bounds__(256, MINB)
     k_bwd3d_ax(float *__restrict__ vol, const float4 *__restrict__ SQ,
                 const __grid_constant__ AxViewParams tab, int nv, float num, float su, float sv,
                 int X, int Y, int Z, int U, int V, int tiles_x, int tiles_y, int tiles_z) {
+    wait_previous();
     const auto param_tab = [&](int j, float4 &p0, float4 &p1, float2 &p2) {
         p0 = tab.p0[j], p1 = tab.p1[j], p2 = tab.p2[j];
     };
@@ -815,17 +826,16 @@ int ensure_plan3d_scratch(Plan3d &p, bool fwd, bool bwd) {
 int launch_forward3d(const Plan3d &p, const float *vol, float *sino, cudaStream_t s) {
     {
         const long long n = (long long)p.volA_elems;
-        k_relayout3d_A<<<ceil_div(n, 256), 256, 0, s>>>(vol, p.X, p.Y, p.Z, p.d_volA);
-        CG_TRY_CUDA(cudaGetLastError());
+        CG_TRY(launch_after(k_relayout3d_A, ceil_div(n, 256), 256, 0, s, 1, vol, p.X, p.Y, p.Z,
+                            p.d_volA));
         dim3 g(ceil_div(p.X + 2 * kP3, 32), ceil_div(p.Z + 2 * kP3, 32), p.Y + 2 * kP3);
-        k_relayout3d_B<<<g, dim3(32, 8), 0, s>>>(vol, p.X, p.Y, p.Z, p.d_volB);
-        CG_TRY_CUDA(cudaGetLastError());
+        CG_TRY(launch_after(k_relayout3d_B, g, dim3(32, 8), 0, s, 1, vol, p.X, p.Y, p.Z,
+                            p.d_volB));
     }
     if (p.nangles > 65535) return set_error(CG_ERR_INVALID, "too many views for one launch");
     dim3 grid(ceil_div(p.U, 32), ceil_div(p.V, 8), p.nangles);
-    k_fwd3d<<<grid, dim3(32, 8), 0, s>>>(p.d_volA, p.d_volB, sino, p.d_forg, p.d_fdu, p.d_fdv,
-                                         p.d_fsrc, p.X, p.Y, p.Z, p.U, p.V, p.exact_t);
-    CG_TRY_CUDA(cudaGetLastError());
+    CG_TRY(launch_after(k_fwd3d, grid, dim3(32, 8), 0, s, 1, p.d_volA, p.d_volB, sino, p.d_forg,
+                        p.d_fdu, p.d_fdv, p.d_fsrc, p.X, p.Y, p.Z, p.U, p.V, p.exact_t));
     return CG_OK;
 }
 
@@ -852,11 +862,10 @@ int launch_forward3d_quad(Plan3d &p, const float *vol, float *sino, cudaStream_t
             return launch_forward3d_tex(p, vol, sino, s);
         }
     }
-    k_relayout3d_qa<<<ceil_div((long long)n, 256), 256, 0, s>>>(vol, p.X, p.Y, p.Z, p.d_volQA);
-    CG_TRY_CUDA(cudaGetLastError());
+    CG_TRY(launch_after(k_relayout3d_qa, ceil_div((long long)n, 256), 256, 0, s, 1, vol, p.X, p.Y,
+                        p.Z, p.d_volQA));
     dim3 g(ceil_div(p.Z + kQP, 32), ceil_div(p.X + kQP, 32), p.Y + kQP);
-    k_relayout3d_qb<<<g, dim3(32, 8), 0, s>>>(vol, p.X, p.Y, p.Z, p.d_volQB);
-    CG_TRY_CUDA(cudaGetLastError());
+    CG_TRY(launch_after(k_relayout3d_qb, g, dim3(32, 8), 0, s, 1, vol, p.X, p.Y, p.Z, p.d_volQB));
     const int utiles = ceil_div(p.U, 32);
     const long long blocks = (long long)utiles * p.nangles * ceil_div(p.V, 8);
     if (blocks >= (1ll << 31)) return set_error(CG_ERR_INVALID, "too many rays for one launch");
@@ -869,10 +878,9 @@ int launch_forward3d_quad(Plan3d &p, const float *vol, float *sino, cudaStream_t
         tex = p.tex3;
     }
     auto kernel = p.fwd_unroll == 2 ? k_fwd3d_quad<2> : k_fwd3d_quad<1>;
-    kernel<<<(unsigned)blocks, 256, 0, s>>>(p.d_volQA, p.d_volQB, sino, p.d_forg, p.d_fdu,
-                                            p.d_fdv, p.d_fsrc, p.X, p.Y, p.Z, p.U, p.V,
-                                            p.nangles, utiles, tex, tex_warps, p.exact_t);
-    CG_TRY_CUDA(cudaGetLastError());
+    CG_TRY(launch_after(kernel, (unsigned)blocks, 256, 0, s, 1, p.d_volQA, p.d_volQB, sino,
+                        p.d_forg, p.d_fdu, p.d_fdv, p.d_fsrc, p.X, p.Y, p.Z, p.U, p.V, p.nangles,
+                        utiles, tex, tex_warps, p.exact_t));
     return CG_OK;
 }
 
@@ -881,9 +889,8 @@ int launch_backward3d(const Plan3d &p, float *vol, const float *sino, cudaStream
     const float hu = (float)(p.U / 2), hv = (float)(p.V / 2);
     if (p.runs_axial()) {
         const long long n = (long long)p.sinoP_elems;
-        k_relayout_sino3d_qd<<<ceil_div(n, 256), 256, 0, s>>>(sino, p.U, p.V, p.nangles,
-                                                              p.d_sinoQ);
-        CG_TRY_CUDA(cudaGetLastError());
+        CG_TRY(launch_after(k_relayout_sino3d_qd, ceil_div(n, 256), 256, 0, s, 1, sino, p.U, p.V,
+                            p.nangles, p.d_sinoQ));
         constexpr int run = 8;
         const int tiles_x = ceil_div(p.X, 32), tiles_y = ceil_div(p.Y, run),
                   tiles_z = ceil_div(p.Z, 8);
@@ -901,11 +908,10 @@ int launch_backward3d(const Plan3d &p, float *vol, const float *sino, cudaStream
                 tab.p1[j] = make_float4(a[3], a[4], a[5], a[6]);
                 tab.p2[j] = make_float2(a[7], a[8]);
             }
-            kernel<<<bricks * 128, 256, 0, s>>>(vol, p.d_sinoQ + plane * c0, tab, nv,
-                                                zplane - p.bsrc[2], p.bsrc[0] + hu - 0.5f,
-                                                p.bsrc[1] + hv - 0.5f, p.X, p.Y, p.Z, p.U, p.V,
-                                                tiles_x, tiles_y, tiles_z);
-            CG_TRY_CUDA(cudaGetLastError());
+            CG_TRY(launch_after(kernel, bricks * 128, 256, 0, s, 1, vol, p.d_sinoQ + plane * c0,
+                                tab, nv, zplane - p.bsrc[2], p.bsrc[0] + hu - 0.5f,
+                                p.bsrc[1] + hv - 0.5f, p.X, p.Y, p.Z, p.U, p.V, tiles_x, tiles_y,
+                                tiles_z));
         }
         return CG_OK;
     }
@@ -913,22 +919,21 @@ int launch_backward3d(const Plan3d &p, float *vol, const float *sino, cudaStream
     {
         const long long n = (long long)p.sinoP_elems;
         if (quad) {
-            k_relayout_sino3d_quad<<<ceil_div(n, 256), 256, 0, s>>>(sino, p.U, p.V, p.nangles,
-                                                                    p.d_sinoQ);
+            CG_TRY(launch_after(k_relayout_sino3d_quad, ceil_div(n, 256), 256, 0, s, 1, sino, p.U,
+                                p.V, p.nangles, p.d_sinoQ));
         } else {
-            k_relayout_sino3d<<<ceil_div(n, 256), 256, 0, s>>>(sino, p.U, p.V, p.nangles,
-                                                               p.d_sinoP);
+            CG_TRY(launch_after(k_relayout_sino3d, ceil_div(n, 256), 256, 0, s, 1, sino, p.U, p.V,
+                                p.nangles, p.d_sinoP));
         }
-        CG_TRY_CUDA(cudaGetLastError());
     }
     const int tiles_x = ceil_div(p.X, 32), tiles_y = ceil_div(p.Y, 8), tiles_z = ceil_div(p.Z, kBZ);
     const int bricks = ceil_div(tiles_x, 2) * ceil_div(tiles_y, 8) * ceil_div(tiles_z, 8);
     // row-pair quads (default), or 8-byte pairs where the quads did not fit
     auto kernel = quad ? k_bwd3d<true, true, true> : k_bwd3d<true, true>;
-    kernel<<<bricks * 128, dim3(32, 8), 0, s>>>(
-        vol, quad ? (const void *)p.d_sinoQ : (const void *)p.d_sinoP, p.d_borg, p.d_bdx,
-        p.d_bdy, p.d_bdz, p.bsrc[0], p.bsrc[1], p.bsrc[2], zplane, hu, hv, p.X, p.Y, p.Z, p.U, p.V, p.nangles, tiles_x, tiles_y, tiles_z);
-    CG_TRY_CUDA(cudaGetLastError());
+    CG_TRY(launch_after(kernel, bricks * 128, dim3(32, 8), 0, s, 1, vol,
+                        quad ? (const void *)p.d_sinoQ : (const void *)p.d_sinoP, p.d_borg,
+                        p.d_bdx, p.d_bdy, p.d_bdz, p.bsrc[0], p.bsrc[1], p.bsrc[2], zplane, hu, hv,
+                        p.X, p.Y, p.Z, p.U, p.V, p.nangles, tiles_x, tiles_y, tiles_z));
     return CG_OK;
 }
 
@@ -943,6 +948,7 @@ namespace {
 
 __global__ void __launch_bounds__(256)
     k_batch3d_qa(const Prob3d *__restrict__ probs, const int *__restrict__ start, int count) {
+    wait_previous();
     const int i = batch_problem(start, count, blockIdx.x);
     const Prob3d &q = probs[i];
     relayout3d_qa_at(q.vol, q.X, q.Y, q.Z, q.QA,
@@ -951,6 +957,7 @@ __global__ void __launch_bounds__(256)
 
 __global__ void __launch_bounds__(256)
     k_batch3d_qb(const Prob3d *__restrict__ probs, const int *__restrict__ start, int count) {
+    wait_previous();
     const int i = batch_problem(start, count, blockIdx.x);
     const Prob3d &q = probs[i];
     const int lin = blockIdx.x - start[i];
@@ -960,6 +967,7 @@ __global__ void __launch_bounds__(256)
 
 __global__ void __launch_bounds__(256, 6)
     k_batch3d_fwd(const Prob3d *__restrict__ probs, const int *__restrict__ start, int count) {
+    wait_previous();
     const int i = batch_problem(start, count, blockIdx.x);
     const Prob3d &q = probs[i];
     fwd3d_quad_block<2>(q.QA, q.QB, q.sino, q.forg, q.fdu, q.fdv, q.fsrc, q.X, q.Y, q.Z, q.U,
@@ -970,6 +978,7 @@ __global__ void __launch_bounds__(256, 6)
 __global__ void __launch_bounds__(256)
     k_batch3d_relayout_sino(const Prob3d *__restrict__ probs, const int *__restrict__ start,
                             int count) {
+    wait_previous();
     const int i = batch_problem(start, count, blockIdx.x);
     const Prob3d &q = probs[i];
     const long long idx = (long long)(blockIdx.x - start[i]) * blockDim.x + threadIdx.x;
@@ -986,6 +995,7 @@ template <int RUN>
 __global__ void __launch_bounds__(256, 5)
     k_batch3d_bwd_ax(const Prob3d *__restrict__ probs, const int *__restrict__ start,
                      int count) {
+    wait_previous();
     const int i = batch_problem(start, count, blockIdx.x);
     const Prob3d &q = probs[i];
     const int lin = blockIdx.x - start[i];
@@ -1004,6 +1014,7 @@ __global__ void __launch_bounds__(256, 5)
 
 __global__ void __launch_bounds__(256, 5)
     k_batch3d_bwd(const Prob3d *__restrict__ probs, const int *__restrict__ start, int count) {
+    wait_previous();
     const int i = batch_problem(start, count, blockIdx.x);
     const Prob3d &q = probs[i];
     bwd3d_block<true, true, true>(q.vol, q.sinoQ, q.borg, q.bdx, q.bdy, q.bdz, q.bsx, q.bsy,
@@ -1098,16 +1109,15 @@ int launch_batch3d_forward(const Prob3d *d_probs, const int *starts,
                            const int totals[kBatch3dStages], int count, cudaStream_t s) {
     const int n1 = count + 1;
     if (totals[0] > 0) {
-        k_batch3d_qa<<<totals[0], 256, 0, s>>>(d_probs, starts, count);
-        CG_TRY_CUDA(cudaGetLastError());
+        CG_TRY(launch_after(k_batch3d_qa, totals[0], 256, 0, s, 1, d_probs, starts, count));
     }
     if (totals[1] > 0) {
-        k_batch3d_qb<<<totals[1], dim3(32, 8), 0, s>>>(d_probs, starts + n1, count);
-        CG_TRY_CUDA(cudaGetLastError());
+        CG_TRY(launch_after(k_batch3d_qb, totals[1], dim3(32, 8), 0, s, 1, d_probs, starts + n1,
+                            count));
     }
     if (totals[2] > 0) {
-        k_batch3d_fwd<<<totals[2], 256, 0, s>>>(d_probs, starts + 2 * n1, count);
-        CG_TRY_CUDA(cudaGetLastError());
+        CG_TRY(launch_after(k_batch3d_fwd, totals[2], 256, 0, s, 1, d_probs, starts + 2 * n1,
+                            count));
     }
     return CG_OK;
 }
@@ -1116,16 +1126,16 @@ int launch_batch3d_backward(const Prob3d *d_probs, const int *starts,
                             const int totals[kBatch3dStages], int count, cudaStream_t s) {
     const int n1 = count + 1;
     if (totals[3] > 0) {
-        k_batch3d_relayout_sino<<<totals[3], 256, 0, s>>>(d_probs, starts + 3 * n1, count);
-        CG_TRY_CUDA(cudaGetLastError());
+        CG_TRY(launch_after(k_batch3d_relayout_sino, totals[3], 256, 0, s, 1, d_probs,
+                            starts + 3 * n1, count));
     }
     if (totals[4] > 0) {
-        k_batch3d_bwd_ax<8><<<totals[4], 256, 0, s>>>(d_probs, starts + 4 * n1, count);
-        CG_TRY_CUDA(cudaGetLastError());
+        CG_TRY(launch_after(k_batch3d_bwd_ax<8>, totals[4], 256, 0, s, 1, d_probs, starts + 4 * n1,
+                            count));
     }
     if (totals[5] > 0) {
-        k_batch3d_bwd<<<totals[5], dim3(32, 8), 0, s>>>(d_probs, starts + 5 * n1, count);
-        CG_TRY_CUDA(cudaGetLastError());
+        CG_TRY(launch_after(k_batch3d_bwd, totals[5], dim3(32, 8), 0, s, 1, d_probs,
+                            starts + 5 * n1, count));
     }
     return CG_OK;
 }
