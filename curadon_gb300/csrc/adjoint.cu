@@ -23,6 +23,12 @@ namespace {
 // QUAD: one float4 per (row, column) of the layout holding the contributions
 // to (row, col), (row, col + 1), (row + 1, col), (row + 1, col + 1), so a
 // sample is one 16-byte atomic instead of two 8-byte ones.
+// A sample's far row is the next one's near row, so while the ray stays in its
+// column the contributions are held in registers: a quad goes out complete
+// every second sample (pairs: every sample).  Bound by the L2's reductions:
+// per call 413 -> 366 us at 513^2 x 437, 3057 -> 2672 at 1024^2 x 1024, 103 ->
+// 92 at 256^2 x 256; pairs 5991 -> 4852 at 2048^2 x 360, 4422 -> 3530 at
+// 1024^2 x 1024.
 template <bool QUAD>
 __device__ __forceinline__ void adj2d_ray(void *__restrict__ accA, void *__restrict__ accB,
                                           const float *__restrict__ sino,
@@ -73,21 +79,59 @@ __device__ __forceinline__ void adj2d_ray(void *__restrict__ accA, void *__restr
     long long ri = (long long)(iq + kPad) * pitch + kPad;  // element of the row start
     const long long rstep = (long long)sq * pitch;
     const float clo = c * (1.f - fq), chi = c * fq;
-    for (int j = 0; j < n; ++j) {
-        const float pf = fminf(fmaxf(floorf(p), -(float)kPad), pmax);
-        const float fp = p - pf;
-        const int ip = (int)pf;
-        // forward: lo = x + fp (y - x) -> weights (1 - fp, fp) on the pair
-        if constexpr (QUAD) {
-            atomicAdd(static_cast<float4 *>(acc) + ri + ip,
-                      make_float4(clo * (1.f - fp), clo * fp, chi * (1.f - fp), chi * fp));
-        } else {
-            float2 *row = static_cast<float2 *>(acc) + ri;
-            atomicAdd(row + ip, make_float2(clo * (1.f - fp), clo * fp));
-            atomicAdd(row + pitch + ip, make_float2(chi * (1.f - fp), chi * fp));
+    // the near row of a sample is the far row of the one before
+    const bool up = sq > 0;
+    const float cn = up ? clo : chi, cf = up ? chi : clo;
+    if constexpr (QUAD) {
+        // held: the last sample's quad, whose far row may still get the next
+        // sample's near row (half: its near row has gone out already)
+        float4 *row = static_cast<float4 *>(acc) + ri;  // element of the sample's lower row
+        float2 near = make_float2(0.f, 0.f), far = near;
+        float4 *at = nullptr;  // the held quad's element
+        bool half = false;
+        int held = 0;
+        auto put = [&] {
+            atomicAdd(at, up ? make_float4(near.x, near.y, far.x, far.y)
+                             : make_float4(far.x, far.y, near.x, near.y));
+        };
+        for (int j = 0; j < n; ++j) {
+            const float pf = fminf(fmaxf(floorf(p), -(float)kPad), pmax);
+            const float fp = p - pf;
+            const int ip = (int)pf;
+            const float2 vn = make_float2(cn * (1.f - fp), cn * fp);
+            const float2 vf = make_float2(cf * (1.f - fp), cf * fp);
+            const bool same = j > 0 && ip == held;
+            if (same && half) {
+                near = make_float2(far.x + vn.x, far.y + vn.y), half = false;
+            } else {
+                if (same) far.x += vn.x, far.y += vn.y;
+                if (j > 0) put();
+                near = same ? make_float2(0.f, 0.f) : vn, half = same;
+            }
+            far = vf, at = row + ip;
+            held = ip;
+            p += vp;
+            row += rstep;
         }
-        p += vp;
-        ri += rstep;
+        if (n > 0) put();
+    } else {
+        float2 *row = static_cast<float2 *>(acc) + ri + (sq > 0 ? 0 : pitch);
+        float2 held = make_float2(0.f, 0.f);
+        int at = -kPad;
+        for (int j = 0; j < n; ++j) {
+            const float pf = fminf(fmaxf(floorf(p), -(float)kPad), pmax);
+            const float fp = p - pf;
+            const int ip = (int)pf;
+            if (ip != at) {
+                if (j > 0) atomicAdd(row + at, held);
+                held = make_float2(0.f, 0.f), at = ip;
+            }
+            atomicAdd(row + ip, make_float2(fmaf(cn, 1.f - fp, held.x), fmaf(cn, fp, held.y)));
+            held = make_float2(cf * (1.f - fp), cf * fp);
+            p += vp;
+            row += rstep;
+        }
+        if (n > 0) atomicAdd(row + at, held);
     }
 }
 
@@ -190,14 +234,16 @@ __global__ void k_fold2d(float *__restrict__ vol, const float2 *__restrict__ A,
 // cells (the quad forward's order): the blocks resident at one time scatter
 // into a slab of the volume's y range, so the atomics stay in L2; otherwise
 // a (U/32, V/8, views) grid of 32 x 8 blocks.
-// MERGE (quads): a sample's upper-slice contribution is held in registers
-// and, when the next sample's lower slice is the same element (the ray
-// advanced one slice within the same row and column), added to it, so the
-// two go out as one atomic.
-// AGG (quads, with MERGE): warp-aggregated atomics -- the lanes of a warp
-// whose lower-slice element coincides at a step (found with
-// __match_any_sync) pass their contributions through shared memory to the
-// lowest such lane, which sums them in lane order and issues one atomic.
+// MERGE (quads): a sample's two quads are held in registers.  The next
+// sample adds to both when it lies in the same cell; when the ray advanced one
+// slice, up or down, within the same row and column, its near quad (the one
+// the ray meets first) is the held far one and both go out as one atomic.
+// Against merging upwards-going rays' slices only: 2446 -> 2116 us at 128^3 x
+// 180, 40.2 -> 33.1 ms at 256^3 x 360, 202 -> 177 us at 64^3 x 90; bound by
+// the L2's reductions as before (16 sectors per warp's atomic), of which a
+// sample now takes 1.4 instead of 1.7.  (Merging across lanes as well was
+// slower: 4.01 ms at 128^3 x 180 -- about 9 % of a warp's same-step targets
+// coincide.)
 // The band-major block `lin`'s cell of this thread.
 __device__ __forceinline__ void adj3d_band_cell(int lin, int utiles, int P, int &iu, int &iv,
                                                 int &view) {
@@ -211,7 +257,7 @@ __device__ __forceinline__ void adj3d_band_cell(int lin, int utiles, int P, int 
 }
 
 // One ray's scatter (the cell (iu, iv) of `view`).
-template <bool QUAD, bool MERGE, bool AGG>
+template <bool QUAD, bool MERGE>
 __device__ __forceinline__ void adj3d_ray(void *__restrict__ A, void *__restrict__ B,
                                           const float *__restrict__ sino,
                                           const float4 *__restrict__ torg,
@@ -260,8 +306,12 @@ __device__ __forceinline__ void adj3d_ray(void *__restrict__ A, void *__restrict
     const float amax = (float)Na, bmax = (float)Y, cmax = (float)Nc;
     const float lo = -(float)kPad;
     float t = tmin;
-    size_t held_at = ~(size_t)0;  // MERGE: element of the held contribution
-    float4 held = make_float4(0.f, 0.f, 0.f, 0.f);
+    // MERGE: the held contributions, of the near slice (the one the ray enters
+    // a cell by) and the far one, and the near one's element
+    const bool down = dc < 0.f;
+    const int slice = pa * pb, ahead = down ? -slice : slice;
+    size_t held_at = ~(size_t)0;
+    float4 near = make_float4(0.f, 0.f, 0.f, 0.f), far = near;
     for (int k = 0; k <= nsteps + 1; ++k) {
         if (!(t <= tmax)) break;
         const float pa_ = fmaf(da, t, sa), pb_ = fmaf(dy, t, s.y), pc_ = fmaf(dc, t, sc);
@@ -274,40 +324,21 @@ __device__ __forceinline__ void adj3d_ray(void *__restrict__ A, void *__restrict
         const float c01 = c * (1.f - wb) * wc, c11 = c * wb * wc;
         if constexpr (QUAD && MERGE) {
             float4 *q = static_cast<float4 *>(L);
-            float4 lower = make_float4(c00 * (1.f - wa), c00 * wa, c10 * (1.f - wa), c10 * wa);
-            const float4 upper =
-                make_float4(c01 * (1.f - wa), c01 * wa, c11 * (1.f - wa), c11 * wa);
-            if (i00 == held_at) {
-                lower.x += held.x, lower.y += held.y, lower.z += held.z, lower.w += held.w;
-            } else if (held_at != ~(size_t)0) {
-                atomicAdd(q + held_at, held);
-            }
-            if constexpr (AGG) {
-                __shared__ float4 s_agg[8][32];
-                const unsigned active = __activemask();
-                const int lane = (int)(threadIdx.x + threadIdx.y * blockDim.x) & 31;
-                const int wslot = (int)(threadIdx.x + threadIdx.y * blockDim.x) >> 5;
-                const unsigned peers = __match_any_sync(active, (unsigned)i00);
-                const int leader = __ffs(peers) - 1;
-                // lanes that share their element with another lane; only
-                // they take part in the exchange and its two warp barriers
-                const unsigned shared = __ballot_sync(active, peers != (1u << lane));
-                if (peers != (1u << lane)) {
-                    if (lane != leader) s_agg[wslot][lane] = lower;
-                    __syncwarp(shared);
-                    if (lane == leader) {
-                        for (unsigned rest = peers & ~(1u << lane); rest; rest &= rest - 1) {
-                            const float4 o = s_agg[wslot][__ffs(rest) - 1];
-                            lower.x += o.x, lower.y += o.y, lower.z += o.z, lower.w += o.w;
-                        }
-                    }
-                    __syncwarp(shared);
-                }
-                if (lane == leader) atomicAdd(q + i00, lower);
+            const float4 lower = make_float4(c00 * (1.f - wa), c00 * wa, c10 * (1.f - wa), c10 * wa);
+            const float4 upper = make_float4(c01 * (1.f - wa), c01 * wa, c11 * (1.f - wa), c11 * wa);
+            const size_t at = down ? i00 + slice : i00;
+            const float4 n1 = down ? upper : lower, f1 = down ? lower : upper;
+            if (at == held_at) {  // the same cell again
+                near.x += n1.x, near.y += n1.y, near.z += n1.z, near.w += n1.w;
+                far.x += f1.x, far.y += f1.y, far.z += f1.z, far.w += f1.w;
             } else {
-                atomicAdd(q + i00, lower);
+                const bool held = held_at != ~(size_t)0, next = at == held_at + ahead;
+                if (held) atomicAdd(q + held_at, near);
+                if (held && !next) atomicAdd(q + (held_at + ahead), far);
+                near = n1;
+                if (next) near.x += far.x, near.y += far.y, near.z += far.z, near.w += far.w;
+                far = f1, held_at = at;
             }
-            held = upper, held_at = i00 + (size_t)pa * pb;
         } else if constexpr (QUAD) {
             float4 *q = static_cast<float4 *>(L) + i00;
             atomicAdd(q, make_float4(c00 * (1.f - wa), c00 * wa, c10 * (1.f - wa), c10 * wa));
@@ -323,11 +354,15 @@ __device__ __forceinline__ void adj3d_ray(void *__restrict__ A, void *__restrict
         t = march_next(t, k, tmin, h, exact_t);
     }
     if constexpr (QUAD && MERGE) {
-        if (held_at != ~(size_t)0) atomicAdd(static_cast<float4 *>(L) + held_at, held);
+        if (held_at != ~(size_t)0) {
+            float4 *q = static_cast<float4 *>(L) + held_at;
+            atomicAdd(q, near);
+            atomicAdd(q + ahead, far);
+        }
     }
 }
 
-template <bool QUAD, bool BAND = false, bool MERGE = false, bool AGG = false>
+template <bool QUAD, bool BAND = false, bool MERGE = false>
 __global__ void __launch_bounds__(256)
     k_adj3d(void *__restrict__ A, void *__restrict__ B, const float *__restrict__ sino,
             const float4 *__restrict__ torg, const float4 *__restrict__ tdu,
@@ -342,8 +377,7 @@ __global__ void __launch_bounds__(256)
         iv = blockIdx.y * blockDim.y + threadIdx.y;
         view = blockIdx.z;
     }
-    adj3d_ray<QUAD, MERGE, AGG>(A, B, sino, torg, tdu, tdv, tsrc, X, Y, Z, U, V, exact_t, iu, iv,
-                                view);
+    adj3d_ray<QUAD, MERGE>(A, B, sino, torg, tdu, tdv, tsrc, X, Y, Z, U, V, exact_t, iu, iv, view);
 }
 
 // vol[z][y][x] += A[z][y][x].x + A[z][y][x-1].y + B[x][y][z].x + B[x][y][z-1].y
@@ -409,8 +443,8 @@ __global__ void __launch_bounds__(256)
     const Prob3d &q = probs[i];
     int iu, iv, view;
     adj3d_band_cell(blockIdx.x - start[i], q.utiles, q.P, iu, iv, view);
-    adj3d_ray<true, true, false>(q.adjA, q.adjB, q.sino, q.forg, q.fdu, q.fdv, q.fsrc, q.X, q.Y,
-                                 q.Z, q.U, q.V, q.exact_t != 0, iu, iv, view);
+    adj3d_ray<true, true>(q.adjA, q.adjB, q.sino, q.forg, q.fdu, q.fdv, q.fsrc, q.X, q.Y, q.Z, q.U,
+                          q.V, q.exact_t != 0, iu, iv, view);
 }
 
 __global__ void __launch_bounds__(256)
@@ -431,7 +465,9 @@ size_t adj2d_quad_elems(const Plan2d &p, bool layoutA) {
 int ensure_adj2d_quads(Plan2d &p) {
     if (p.d_quadA) return CG_OK;
     CG_TRY_CUDA(cudaMalloc(&p.d_quadA, adj2d_quad_elems(p, true) * sizeof(float4)));
-    CG_TRY_CUDA(cudaMalloc(&p.d_quadB, adj2d_quad_elems(p, false) * sizeof(float4)));
+    const cudaError_t e = cudaMalloc(&p.d_quadB, adj2d_quad_elems(p, false) * sizeof(float4));
+    if (e != cudaSuccess) cudaFree(p.d_quadA), p.d_quadA = nullptr;
+    CG_TRY_CUDA(e);
     return CG_OK;
 }
 
@@ -454,8 +490,19 @@ int launch_adjoint2d(Plan2d &p, float *vol, const float *sino, cudaStream_t s) {
     dim3 grid(ceil_div(p.det, p.fwd_bx), ceil_div(p.nangles, p.fwd_by));
     if (grid.y > 65535) return set_error(CG_ERR_INVALID, "too many views for one launch");
     const dim3 fgrid(ceil_div(p.W, 32), ceil_div(p.H, 8));
-    // quad accumulators when both fit in 96 MB, where the L2 holds the atomics
-    if (p.adj_quad > 0 || (p.adj_quad < 0 && (na + nb) * sizeof(float4) <= (96u << 20))) {
+    // quad accumulators up to 160 MB (2230^2), a little above what the L2 can
+    // hold: quads / pairs, us: 1448^2 x 1024 5235 / 6695, 2048^2 x 360 3842 /
+    // 4864, 3000^2 x 360 10698 / 10162, 4096^2 x 180 15771 / 11110.  A plan
+    // that gets no room for them (or is first used under capture, where nothing
+    // may be allocated) scatters into pairs, which every plan has
+    bool quad = p.adj_quad > 0;
+    if (p.adj_quad < 0 && (na + nb) * sizeof(float4) <= (160u << 20)) {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        if (!p.d_quadA) CG_TRY_CUDA(cudaStreamIsCapturing(s, &capture));
+        quad = capture == cudaStreamCaptureStatusNone && ensure_adj2d_quads(p) == CG_OK;
+        if (!quad) clear_error();
+    }
+    if (quad) {
         if (int rc = ensure_adj2d_quads(p)) return rc;
         CG_TRY_CUDA(cudaMemsetAsync(p.d_quadA, 0, na * sizeof(float4), s));
         CG_TRY_CUDA(cudaMemsetAsync(p.d_quadB, 0, nb * sizeof(float4), s));
@@ -526,10 +573,8 @@ int launch_adjoint3d(Plan3d &p, float *vol, const float *sino, cudaStream_t s) {
         if (int rc = ensure_adj3d_quads(p)) return rc;
         CG_TRY_CUDA(cudaMemsetAsync(p.d_quadA, 0, elems * sizeof(float4), s));
         CG_TRY_CUDA(cudaMemsetAsync(p.d_quadB, 0, elems * sizeof(float4), s));
-        auto kq = p.adj_agg   ? (band ? k_adj3d<true, true, true, true>
-                                      : k_adj3d<true, false, true, true>)
-                  : p.adj_merge ? (band ? k_adj3d<true, true, true> : k_adj3d<true, false, true>)
-                                : (band ? k_adj3d<true, true> : k_adj3d<true, false>);
+        auto kq = p.adj_merge ? (band ? k_adj3d<true, true, true> : k_adj3d<true, false, true>)
+                              : (band ? k_adj3d<true, true> : k_adj3d<true, false>);
         CG_TRY(launch_after(kq, grid, dim3(32, 8), 0, s, 1, p.d_quadA, p.d_quadB, sino, p.d_forg,
                             p.d_fdu, p.d_fdv, p.d_fsrc, p.X, p.Y, p.Z, p.U, p.V, p.nangles, utiles,
                             p.exact_t));

@@ -82,7 +82,7 @@ bool listed(const int (&list)[N], int v) {
 // quads or on 8-byte pairs, its fallback where quads do not fit) | ax8m5
 // (axial runs);
 // adj3d = pair | quad; adj3d_order = band | view; adj3d_merge = 0 | 1;
-// adj3d_agg = 0 | 1 (warp-aggregated atomics on the merged quads);
+// (adj3d_agg, once atomics merged across lanes, is ignored);
 // t3d = step | exact (running-sum or drift-free sample parameters of the 3D
 // ray marches).  Unknown tokens are ignored; without the variable every plan
 // starts at the measured defaults.
@@ -155,7 +155,6 @@ void apply_algo_env(Plan2d *p2, Plan3d *p3) {
             if (val == "step") p3->exact_t = false;
             if (val == "exact") p3->exact_t = true;
         }
-        if (p3 && key == "adj3d_agg") p3->adj_agg = val == "1";
         if (p3 && key == "adj3d_merge") {
             if (val == "0") p3->adj_merge = false;
             if (val == "1") p3->adj_merge = true;

@@ -250,12 +250,9 @@ struct Plan3d {
     // block order of the scatter: -1 band-major when the accumulators exceed
     // 96 MB (they no longer stay in L2), else view-major; 1 / 0 forced
     int adj_band = -1;
-    // merge consecutive samples' shared quad element into one atomic
-    // (-11 % at 128^3, -10 % at 256^3)
+    // hold consecutive samples' quads and send shared ones as one atomic
+    // (-26 % at 128^3, -23 % at 256^3)
     bool adj_merge = true;
-    // merged quads plus warp-aggregated atomics (lanes whose lower-slice
-    // element coincides combine before one atomic)
-    bool adj_agg = false;
     // ray-march sample parameters t_k = tmin + k h by one FMA instead of the
     // reference's running sum t += h, whose rounding accumulates along long
     // rays (on from 512 voxels along an axis: against the FP64 oracle the
