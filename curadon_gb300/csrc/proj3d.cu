@@ -363,16 +363,24 @@ __device__ __forceinline__ Ray3 setup_ray3(const float4 o, const float4 du, cons
 // need no clamp).  With tex_warps > 0 (algorithm 5) the first tex_warps
 // warps of each block take their rays through the texture unit instead
 // (the reference's tex3D sampling): the texture path and the L1 load path
-// then work side by side (3 of 8 warps: -8 % at 256^3, -21 % at 512^3
-// against quads alone).
-// UNR = 2 (default): two samples per iteration, both samples' loads (or
-// texture fetches) issued before either is accumulated, so each warp keeps
-// twice the memory requests in flight; the samples, their order of
-// summation and the march's parameter sequence are those of UNR = 1, so the
-// results are the same bits (the second sample's loads happen even when it
-// lies past tmax, at an offset clamped into the array, and are then
-// dropped).  -2 % at 256^3, -0.7 % at 512^3 (the texture warps gain; the
-// quads alone do not change; four fetches per iteration: no better).
+// then work side by side.  Their lanes run over the patch in 2 x 4 cells at a
+// time, the quad warps' in rows of 8: the texture unit's four-lane groups like
+// compact footprints, the 16-byte loads long rows (texture warps in rows of 8:
+// 13.0 ms at 256^3 and 57.9 at 512^3 x 180; quad warps in 2 x 4: 12.3 and 50.2;
+// each its own way: 11.7 and 49.5).
+// Bound by the L1's data pipe (two 16-byte loads a sample, 5.3 wavefronts
+// each).  While the ray advances a slice a step within its row and column, a
+// sample's near quad is the far quad of the sample before and is not loaded
+// again: 15.32 -> 13.98 ms at 256^3 x 360 without texture warps, 13.85 -> 13.0
+// with three of eight.  The quad warps take one sample at a time (two: 48
+// registers, five blocks per SM, 13.4 ms against 13.0 at 40 and six).
+// UNR = 3 (default): the texture warps issue three fetches before the first is
+// accumulated; the samples, their order of summation and the march's parameter
+// sequence are those of UNR = 1, so the results are the same bits (fetches past
+// tmax are dropped).  1: 13.66 ms, 2: 13.01, 3: 12.97, 4: 12.99 (with the
+// lanes in rows of 8).
+// In all, per call: 926 -> 797 us at 128^3 x 180, 13.85 -> 11.64 ms at 256^3 x
+// 360, 60.0 -> 48.6 at 512^3 x 180.
 // Block `lin` of the launch order above (the batched forward passes each
 // problem's own block index).
 template <int UNR>
@@ -384,12 +392,14 @@ __device__ __forceinline__ void fwd3d_quad_block(
     const int ut = lin % utiles, rest = lin / utiles;
     const int view = rest % P, band = rest / P;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int iu = ut * 32 + (warp & 3) * 8 + (lane & 7);
-    const int iv = band * 8 + (warp >> 2) * 4 + (lane >> 3);
+    const bool texture = warp < tex_warps;
+    const int pu = texture ? (lane & 1) + (lane >> 2 & 6) : lane & 7;
+    const int pv = texture ? lane >> 1 & 3 : lane >> 3;
+    const int iu = ut * 32 + (warp & 3) * 8 + pu, iv = band * 8 + (warp >> 2) * 4 + pv;
     if (iu >= U || iv >= V) return;
     const Ray3 r = setup_ray3(torg[view], tdu[view], tdv[view], tsrc[view], iu, iv, X, Y, Z);
     if (!r.hit) return;
-    if (warp < tex_warps) {
+    if (texture) {
         // this warp's rays through the texture unit (trilinear, 8-bit weights)
         // UNR fetches per iteration (their sample parameters in sequence),
         // accumulated in order up to the first one past tmax
@@ -431,56 +441,44 @@ __device__ __forceinline__ void fwd3d_quad_block(
     const unsigned base = 0x4B400000u - (unsigned)kP3;
     // off = (bits_c - base) slice + (bits_b - base) PA + (bits_a - base), mod 2^32
     const unsigned K = base * slice + base * PA + base;
-    const float4 *Q1 = Q + slice;
-    // one sample at parameter t: its two quads' loads, then its value
-    struct Fetch {
-        float4 q0, q1;
-        float wa, wb, wc;
-    };
-    auto fetch = [&](float t) {
-        Fetch f;
+    // a sample's near quad (of the slice the ray meets first) is the far one of
+    // the sample before when the ray advanced one slice within its row and
+    // column
+    const bool down = dc < 0.f;
+    const unsigned ahead = down ? 0u - slice : slice;
+    const float4 *Qn = down ? Q + slice : Q, *Qf = down ? Q : Q + slice;
+    // the sample before: its offset (none: matches no offset) and far quad
+    unsigned last = ~0u - ahead;
+    float4 far = make_float4(0.f, 0.f, 0.f, 0.f);
+    float acc = 0.f, t = r.tmin;
+    const int kend = r.nsteps + 2;
+    for (int k = 0; k < kend; ++k) {
+        if (!(t <= r.tmax)) break;
         const float pa = fmaf(da, t, sa), pb = fmaf(r.dy, t, r.sy), pc = fmaf(dc, t, sc);
         const float ta = __fadd_rd(pa, kMagic), tb = __fadd_rd(pb, kMagic),
                     tc = __fadd_rd(pc, kMagic);
-        f.wa = __fadd_rn(pa, -__fadd_rn(ta, -kMagic));
-        f.wb = __fadd_rn(pb, -__fadd_rn(tb, -kMagic));
-        f.wc = __fadd_rn(pc, -__fadd_rn(tc, -kMagic));
+        const float wa = __fadd_rn(pa, -__fadd_rn(ta, -kMagic));
+        const float wb = __fadd_rn(pb, -__fadd_rn(tb, -kMagic));
+        const float wc = __fadd_rn(pc, -__fadd_rn(tc, -kMagic));
         unsigned off = __float_as_uint(tc) * slice + __float_as_uint(tb) * PA +
                        (__float_as_uint(ta) - K);
         off = min(off, maxoff);
-        f.q0 = __ldg(Q + off), f.q1 = __ldg(Q1 + off);
-        return f;
-    };
-    auto value = [](const Fetch &f) {
-        const float l0 = fmaf(f.wa, f.q0.y, f.q0.x), g0 = fmaf(f.wa, f.q0.w, f.q0.z);
-        const float l1 = fmaf(f.wa, f.q1.y, f.q1.x), g1 = fmaf(f.wa, f.q1.w, f.q1.z);
-        const float m0 = fmaf(f.wb, g0, l0), m1 = fmaf(f.wb, g1, l1);
-        return fmaf(f.wc, m1 - m0, m0);
-    };
-    // the quads: two samples per iteration whenever UNR >= 2
-    constexpr int QU = UNR >= 2 ? 2 : 1;
-    float acc = 0.f, t = r.tmin;
-    const int kend = r.nsteps + 2;
-    for (int k = 0; k < kend; k += QU) {
-        if (!(t <= r.tmax)) break;
-        const Fetch f0 = fetch(t);
-        if constexpr (QU == 2) {
-            const float t1 = march_next(t, k, r.tmin, r.h, exact_t);
-            const Fetch f1 = fetch(t1);
-            acc += value(f0);
-            if (!(k + 1 < kend && t1 <= r.tmax)) break;
-            acc += value(f1);
-            t = march_next(t1, k + 1, r.tmin, r.h, exact_t);
-        } else {
-            acc += value(f0);
-            t = march_next(t, k, r.tmin, r.h, exact_t);
-        }
+        float4 near = far;
+        if (off != last + ahead) near = __ldg(Qn + off);
+        far = __ldg(Qf + off);
+        last = off;
+        const float ln = fmaf(wa, near.y, near.x), gn = fmaf(wa, near.w, near.z);
+        const float lf = fmaf(wa, far.y, far.x), gf = fmaf(wa, far.w, far.z);
+        const float mn = fmaf(wb, gn, ln), mf = fmaf(wb, gf, lf);
+        const float m0 = down ? mf : mn, m1 = down ? mn : mf;
+        acc += fmaf(wc, m1 - m0, m0);
+        t = march_next(t, k, r.tmin, r.h, exact_t);
     }
     sino[((size_t)view * V + iv) * U + iu] = acc;
 }
 
 template <int UNR>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 6)
     k_fwd3d_quad(const float4 *__restrict__ QA, const float4 *__restrict__ QB,
                  float *__restrict__ sino, const float4 *__restrict__ torg,
                  const float4 *__restrict__ tdu, const float4 *__restrict__ tdv,
@@ -877,7 +875,7 @@ int launch_forward3d_quad(Plan3d &p, const float *vol, float *sino, cudaStream_t
         if (rc) return rc;
         tex = p.tex3;
     }
-    auto kernel = p.fwd_unroll == 2 ? k_fwd3d_quad<2> : k_fwd3d_quad<1>;
+    auto kernel = p.fwd_unroll == 2 ? k_fwd3d_quad<3> : k_fwd3d_quad<1>;
     CG_TRY(launch_after(kernel, (unsigned)blocks, 256, 0, s, 1, p.d_volQA, p.d_volQB, sino,
                         p.d_forg, p.d_fdu, p.d_fdv, p.d_fsrc, p.X, p.Y, p.Z, p.U, p.V, p.nangles,
                         utiles, tex, tex_warps, p.exact_t));
@@ -970,7 +968,7 @@ __global__ void __launch_bounds__(256, 6)
     wait_previous();
     const int i = batch_problem(start, count, blockIdx.x);
     const Prob3d &q = probs[i];
-    fwd3d_quad_block<2>(q.QA, q.QB, q.sino, q.forg, q.fdu, q.fdv, q.fsrc, q.X, q.Y, q.Z, q.U,
+    fwd3d_quad_block<3>(q.QA, q.QB, q.sino, q.forg, q.fdu, q.fdv, q.fsrc, q.X, q.Y, q.Z, q.U,
                         q.V, q.P, q.utiles, q.tex, q.tex_warps, q.exact_t != 0,
                         blockIdx.x - start[i]);
 }
