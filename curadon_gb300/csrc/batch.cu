@@ -50,6 +50,7 @@ struct cg_batch2d {
     int *d_sorted_starts[2] = {};
     int active = 0;           // problems [0, active) run (cg_batch2d_set_active)
     bool adjoint_ready = false;  // the plans' quad accumulators are bound
+    cg::SideStream side;         // of the highest priority (no stream: all work in turn)
 
     // blocks of each stage for the active problems
     void active_totals(int out[cg::kBatchStages]) const {
@@ -82,6 +83,25 @@ using namespace cg;
 
 namespace {
 
+void free_side(SideStream &x) {
+    if (x.fork) cudaEventDestroy(x.fork);
+    if (x.join) cudaEventDestroy(x.join);
+    if (x.stream) cudaStreamDestroy(x.stream);
+    x = SideStream{};
+}
+
+// A side stream of the highest priority, or none where it cannot be had.
+void make_side(SideStream &x) {
+    int low = 0, high = 0;
+    if (cudaDeviceGetStreamPriorityRange(&low, &high) != cudaSuccess ||
+        cudaStreamCreateWithPriority(&x.stream, cudaStreamNonBlocking, high) != cudaSuccess ||
+        cudaEventCreateWithFlags(&x.fork, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&x.join, cudaEventDisableTiming) != cudaSuccess) {
+        (void)cudaGetLastError();
+        free_side(x);
+    }
+}
+
 void free_batch(cg_batch2d *b) {
     if (b->d_probs) cudaFree(b->d_probs);
     if (b->d_starts) cudaFree(b->d_starts);
@@ -89,6 +109,7 @@ void free_batch(cg_batch2d *b) {
         if (b->d_sorted[k]) cudaFree(b->d_sorted[k]);
         if (b->d_sorted_starts[k]) cudaFree(b->d_sorted_starts[k]);
     }
+    free_side(b->side);
 }
 
 // The work list of a batch in the given order of its problems, on the device.
@@ -201,6 +222,7 @@ int cg_batch2d_create(cg_batch2d **batch, cg_plan2d *const *plans, float *const 
         if ((e = upload_work(*b, order, &b->d_sorted[k], &b->d_sorted_starts[k])) != cudaSuccess)
             return fail(e);
     }
+    make_side(b->side);
     *batch = b.release();
     return CG_OK;
 }
@@ -230,7 +252,9 @@ int cg_batch2d_forward(cg_batch2d *batch, void *stream) {
         return launch_batch2d_fwd_tex(probs, starts, totals, batch->count, 13, 1,
                                       (cudaStream_t)stream);
     if (batch->fwd_algo == 2)
-        return launch_batch2d_fwd_plans(probs, starts, totals, batch->count, (cudaStream_t)stream);
+        return launch_batch2d_fwd_plans(probs, starts, totals, batch->count,
+                                        batch->side.stream ? &batch->side : nullptr,
+                                        (cudaStream_t)stream);
     return launch_batch2d(probs, starts, totals, batch->count, true, (cudaStream_t)stream);
 }
 

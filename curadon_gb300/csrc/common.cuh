@@ -312,6 +312,13 @@ int widen_half(const void *in, float *out, long long n, cudaStream_t s);
 int narrow_to_half(const float *in, void *out, long long n, cudaStream_t s);
 int add_into_half(void *vol, const float *add, long long n, cudaStream_t s);
 
+// A stream for work beside the caller's, and the events that fork it from the
+// caller's stream and join it again.
+struct SideStream {
+    cudaStream_t stream = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
+};
+
 int launch_relayout_sino2d(const Plan2d &p, const float *sino, cudaStream_t s);
 // batches (proj2d.cu): blocks of each stage of one problem, and the launch of
 // one direction over a batch whose starts hold 4 x (count + 1) block starts
@@ -329,7 +336,8 @@ int launch_batch2d_adjoint(const Prob2d *probs, const int *starts,
 // the "plans" forward: texture rays of the problems that are not chunked
 // (stages 14 and 9) and the chunked bundles of the others (stages 7 and 8)
 int launch_batch2d_fwd_plans(const Prob2d *d_probs, const int *starts,
-                             const int totals[kBatchStages], int count, cudaStream_t s);
+                             const int totals[kBatchStages], int count, const SideStream *side,
+                             cudaStream_t s);
 // the texture forward of the stages `fill` (arrays) and `rays` (tiles)
 int launch_batch2d_fwd_tex(const Prob2d *d_probs, const int *starts,
                            const int totals[kBatchStages], int count, int fill, int rays,

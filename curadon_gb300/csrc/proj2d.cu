@@ -1705,18 +1705,36 @@ bool batch_chunked(const Plan2d &p) {
            std::max(p.pitchA(), p.pitchB()) < 32768;
 }
 
+// The chunked problems run beside the texture ones, on the batch's side stream
+// of the highest priority: their bundles load through the L1, the texture rays
+// through the texture unit, whose blocks fill what the bundles (three per SM,
+// all its registers) leave and their tail.  One after the other / so, us: 12
+// problems of 192^2 .. 1024^2 1469 / 1331, 4 791 / 745, 6 991 / 847, 16 1640 /
+// 1515 (without the priority 1442, 785, 990, 1576: the texture rays, launched
+// first, fill the SMs).
 int launch_batch2d_fwd_plans(const Prob2d *d_probs, const int *starts,
-                             const int totals[kBatchStages], int count, cudaStream_t s) {
-    int rc = launch_batch2d_fwd_tex(d_probs, starts, totals, count, 14, 9, s);
-    if (rc) return rc;
-    if (totals[8] == 0) return CG_OK;
-    CG_TRY(launch_after(k_batch_relayout2d_abs, totals[7], dim3(32, 8), 0, s, 1, d_probs,
-                        starts + 7 * (count + 1), count));
+                             const int totals[kBatchStages], int count, const SideStream *side,
+                             cudaStream_t s) {
+    if (totals[8] == 0) return launch_batch2d_fwd_tex(d_probs, starts, totals, count, 14, 9, s);
     const size_t smem = cslab_smem(kCsCols);
-    if ((rc = ensure_smem_attr((const void *)k_batch_fwd2d_cslab, (int)smem))) return rc;
-    CG_TRY(launch_after(k_batch_fwd2d_cslab, totals[8], 256, smem, s, 1, d_probs,
-                        starts + 8 * (count + 1), count));
-    return CG_OK;
+    CG_TRY(ensure_smem_attr((const void *)k_batch_fwd2d_cslab, (int)smem));
+    const bool fork = side && totals[9] > 0;
+    const cudaStream_t cs = fork ? side->stream : s;
+    if (fork) {
+        CG_TRY_CUDA(cudaEventRecord(side->fork, s));
+        CG_TRY_CUDA(cudaStreamWaitEvent(cs, side->fork, 0));
+    }
+    int rc = launch_after(k_batch_relayout2d_abs, totals[7], dim3(32, 8), 0, cs, 1, d_probs,
+                          starts + 7 * (count + 1), count);
+    if (!rc)
+        rc = launch_after(k_batch_fwd2d_cslab, totals[8], 256, smem, cs, 1, d_probs,
+                          starts + 8 * (count + 1), count);
+    if (!rc) rc = launch_batch2d_fwd_tex(d_probs, starts, totals, count, 14, 9, s);
+    if (fork) {  // the caller's stream goes on when both are done
+        CG_TRY_CUDA(cudaEventRecord(side->join, cs));
+        CG_TRY_CUDA(cudaStreamWaitEvent(s, side->join, 0));
+    }
+    return rc;
 }
 
 int launch_batch2d(const Prob2d *probs, const int *starts, const int totals[kBatchStages],
