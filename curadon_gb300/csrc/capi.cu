@@ -768,18 +768,28 @@ int cg_plan2d_tables(const cg_plan2d *plan, float *sources, float *u_origins, fl
 
 namespace {
 
-int forward2d_f32(cg_plan2d *plan, const float *volume, float *sinogram, cudaStream_t s) {
-    if (plan->algo_fwd == 1) return launch_forward2d_tex(*plan, volume, sinogram, s);
-    int rc = launch_relayout2d(*plan, volume, s);
+// FP32 sums from an FP32 or half input (`half`), which the kernels that lay it
+// out read as it is.
+int forward2d(cg_plan2d *plan, const void *volume, bool half, float *sinogram, cudaStream_t s) {
+    if (plan->algo_fwd == 1) return launch_forward2d_tex(*plan, volume, half, sinogram, s);
+    int rc = launch_relayout2d(*plan, volume, half, s);
     if (rc) return rc;
     if (plan->algo_fwd == 4) return launch_forward2d_cslab(*plan, sinogram, s, plan->fwd_chunk_rows);
     return launch_forward2d(*plan, sinogram, s);
 }
 
-int backward2d_f32(cg_plan2d *plan, float *volume, const float *sinogram, cudaStream_t s) {
-    if (plan->algo_bwd == 1) return launch_backward2d_tex(*plan, volume, sinogram, s);
-    if (plan->algo_bwd == 2) return launch_backward2d_smem(*plan, volume, sinogram, s);
-    int rc = launch_relayout_sino2d(*plan, sinogram, s);
+int backward2d(cg_plan2d *plan, float *volume, const void *sinogram, bool half, cudaStream_t s) {
+    if (plan->algo_bwd == 1) {  // a copy into the texture's array: FP32 only
+        if (half) {
+            if (int rc = ensure_half_scratch(*plan, false, true)) return rc;
+            const long long n = (long long)plan->det * plan->nangles;
+            if (int rc = widen_half(sinogram, plan->d_sino32, n, s)) return rc;
+            sinogram = plan->d_sino32;
+        }
+        return launch_backward2d_tex(*plan, volume, (const float *)sinogram, s);
+    }
+    if (plan->algo_bwd == 2) return launch_backward2d_smem(*plan, volume, sinogram, half, s);
+    int rc = launch_relayout_sino2d(*plan, sinogram, half, s);
     if (rc) return rc;
     return launch_backward2d(*plan, volume, s);
 }
@@ -796,18 +806,11 @@ int cg_forward_2d_ex(cg_plan2d *plan, const void *volume, void *sinogram, int si
     CG_REQUIRE(guard.ok(), "cannot select the plan's device");
     cudaStream_t s = (cudaStream_t)stream;
     const bool hv = plan->vol_bits == 16, hs = sino_bits == 16;
-    if (!hv && !hs) return forward2d_f32(plan, (const float *)volume, (float *)sinogram, s);
-    int rc = ensure_half_scratch(*plan, hv, hs);
+    if (!hs) return forward2d(plan, volume, hv, (float *)sinogram, s);
+    int rc = ensure_half_scratch(*plan, false, true);
     if (rc) return rc;
-    const float *vol = (const float *)volume;
-    if (hv) {
-        if ((rc = widen_half(volume, plan->d_vol32, (long long)plan->W * plan->H, s))) return rc;
-        vol = plan->d_vol32;
-    }
-    float *sino = hs ? plan->d_sino32 : (float *)sinogram;
-    if ((rc = forward2d_f32(plan, vol, sino, s))) return rc;
-    if (hs) return narrow_to_half(sino, sinogram, (long long)plan->det * plan->nangles, s);
-    return CG_OK;
+    if ((rc = forward2d(plan, volume, hv, plan->d_sino32, s))) return rc;
+    return narrow_to_half(plan->d_sino32, sinogram, (long long)plan->det * plan->nangles, s);
 }
 
 int cg_backward_2d_ex(cg_plan2d *plan, void *volume, const void *sinogram, int sino_bits,
@@ -820,19 +823,12 @@ int cg_backward_2d_ex(cg_plan2d *plan, void *volume, const void *sinogram, int s
     CG_REQUIRE(guard.ok(), "cannot select the plan's device");
     cudaStream_t s = (cudaStream_t)stream;
     const bool hv = plan->vol_bits == 16, hs = sino_bits == 16;
-    if (!hv && !hs) return backward2d_f32(plan, (float *)volume, (const float *)sinogram, s);
-    int rc = ensure_half_scratch(*plan, hv, hs);
+    if (!hv) return backward2d(plan, (float *)volume, sinogram, hs, s);
+    int rc = ensure_half_scratch(*plan, true, false);
     if (rc) return rc;
-    const float *sino = (const float *)sinogram;
-    if (hs) {
-        const long long n = (long long)plan->det * plan->nangles;
-        if ((rc = widen_half(sinogram, plan->d_sino32, n, s))) return rc;
-        sino = plan->d_sino32;
-    }
-    if (!hv) return backward2d_f32(plan, (float *)volume, sino, s);
     const long long nv = (long long)plan->W * plan->H;
     CG_TRY_CUDA(cudaMemsetAsync(plan->d_vol32, 0, sizeof(float) * nv, s));
-    if ((rc = backward2d_f32(plan, plan->d_vol32, sino, s))) return rc;
+    if ((rc = backward2d(plan, plan->d_vol32, sinogram, hs, s))) return rc;
     return add_into_half(volume, plan->d_vol32, nv, s);
 }
 

@@ -2,6 +2,7 @@
 // shared by the sm_103a projection kernels.
 #pragma once
 
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -294,7 +295,8 @@ void free_plan3d(Plan3d *p);
 // ------------------------------------------------------------ kernels
 
 int launch_plan2d_tables(Plan2d &p, cudaStream_t s);
-int launch_relayout2d(const Plan2d &p, const float *vol, cudaStream_t s);
+// (vol and sino of FP32 or half values)
+int launch_relayout2d(const Plan2d &p, const void *vol, bool half, cudaStream_t s);
 // Reads and clears the count of bounded waits that gave up in this
 // library's kernels on the current device (cg_wait_timeouts).
 int take_wait_timeouts(unsigned long long *count);
@@ -319,7 +321,7 @@ struct SideStream {
     cudaEvent_t fork = nullptr, join = nullptr;
 };
 
-int launch_relayout_sino2d(const Plan2d &p, const float *sino, cudaStream_t s);
+int launch_relayout_sino2d(const Plan2d &p, const void *sino, bool half, cudaStream_t s);
 // batches (proj2d.cu): blocks of each stage of one problem, and the launch of
 // one direction over a batch whose starts hold 4 x (count + 1) block starts
 void batch_blocks(const Plan2d &p, int blocks[kBatchStages]);
@@ -353,7 +355,8 @@ int launch_adjoint2d(Plan2d &p, float *vol, const float *sino, cudaStream_t s);
 int launch_adjoint3d(Plan3d &p, float *vol, const float *sino, cudaStream_t s);
 
 // the staged backprojection (with the sinogram's re-layout where it reads it)
-int launch_backward2d_smem(const Plan2d &p, float *vol, const float *sino, cudaStream_t s);
+int launch_backward2d_smem(const Plan2d &p, float *vol, const void *sino, bool half,
+                           cudaStream_t s);
 // blocks of the quarter-turn backprojection of a W x W image
 int sym_quadrant_blocks(int W);
 // views whose sum the staged backprojection adds to the volume at a time
@@ -365,7 +368,7 @@ int launch_forward2d_cslab(const Plan2d &p, float *sino, cudaStream_t s, int row
 int tex_blocks(const Plan2d &p);
 // The plan's 2D volume texture array and object (allocated once).
 int ensure_vol_texture(Plan2d &p);
-int launch_forward2d_tex(Plan2d &p, const float *vol, float *sino, cudaStream_t s);
+int launch_forward2d_tex(Plan2d &p, const void *vol, bool half, float *sino, cudaStream_t s);
 int launch_backward2d_tex(Plan2d &p, float *vol, const float *sino, cudaStream_t s);
 // texture forward (tex3D, the reference's trilinear sampling)
 int launch_forward3d_tex(Plan3d &p, const float *vol, float *sino, cudaStream_t s);
@@ -414,6 +417,10 @@ int launch_after(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, 
 }
 #ifdef __CUDACC__
 __device__ __forceinline__ void wait_previous() { cudaGridDependencySynchronize(); }
+
+// A stored value, FP32 or half, in FP32.
+__device__ __forceinline__ float to_float(float v) { return v; }
+__device__ __forceinline__ float to_float(__half v) { return __half2float(v); }
 #endif
 
 // Reads CURADON_GB300_ALGO ("fwd2d=tex,bwd2d=smem,fwd3d=tex2l,...") over the

@@ -84,8 +84,8 @@ constexpr int kTile = 32;
 // ABS: the pairs (v[c] - (c - C) d[c], d[c]) with C = W / 2 (layA) or H / 2
 // (layB), so that the linear sample at column coordinate p is e + (p - C) d
 // with no fraction to form (the chunked forward's absolute-position form).
-template <bool ABS = false>
-__device__ __forceinline__ void relayout2d_tile(const float *__restrict__ vol, int W, int H,
+template <bool ABS = false, class T>
+__device__ __forceinline__ void relayout2d_tile(const T *__restrict__ vol, int W, int H,
                                                 float2 *__restrict__ A, float2 *__restrict__ B,
                                                 int pa, int pb, int bx, int by) {
     __shared__ float tile[kTile + 1][kTile + 1];
@@ -93,7 +93,8 @@ __device__ __forceinline__ void relayout2d_tile(const float *__restrict__ vol, i
     for (int j = threadIdx.y; j < kTile + 1; j += blockDim.y)
         for (int i = threadIdx.x; i < kTile + 1; i += blockDim.x) {
             const int x = x0 + i, y = y0 + j;
-            tile[j][i] = (x >= 0 && x < W && y >= 0 && y < H) ? vol[(size_t)y * W + x] : 0.f;
+            tile[j][i] =
+                (x >= 0 && x < W && y >= 0 && y < H) ? to_float(vol[(size_t)y * W + x]) : 0.f;
         }
     __syncthreads();
     const int tx = threadIdx.x;
@@ -115,9 +116,9 @@ __device__ __forceinline__ void relayout2d_tile(const float *__restrict__ vol, i
     }
 }
 
-template <bool ABS>
+template <bool ABS, class T>
 __global__ void __launch_bounds__(256)
-    k_relayout2d(const float *__restrict__ vol, int W, int H, float2 *__restrict__ A,
+    k_relayout2d(const T *__restrict__ vol, int W, int H, float2 *__restrict__ A,
                  float2 *__restrict__ B, int pa, int pb) {
     wait_previous();
     relayout2d_tile<ABS>(vol, W, H, A, B, pa, pb, blockIdx.x, blockIdx.y);
@@ -125,23 +126,23 @@ __global__ void __launch_bounds__(256)
 
 // ABS: (t[k] - (k - det / 2) d[k], d[k]), the staged backprojector's
 // absolute-position form (a sample at cell coordinate u is e + (u - det / 2) d).
-template <bool ABS = false>
-__device__ __forceinline__ void relayout_sino2d_elem(const float *__restrict__ sino, int det,
+template <bool ABS = false, class T>
+__device__ __forceinline__ void relayout_sino2d_elem(const T *__restrict__ sino, int det,
                                                      int nangles, float2 *__restrict__ S,
                                                      long long idx) {
     const int pitch = det + 2 * kPad;
     if (idx >= (long long)pitch * nangles) return;
     const int a = (int)(idx / pitch);
     const int k = (int)(idx % pitch) - kPad;
-    const float *row = sino + (size_t)a * det;
-    const float t0 = (k >= 0 && k < det) ? row[k] : 0.f;
-    const float t1 = (k + 1 >= 0 && k + 1 < det) ? row[k + 1] : 0.f;
+    const T *row = sino + (size_t)a * det;
+    const float t0 = (k >= 0 && k < det) ? to_float(row[k]) : 0.f;
+    const float t1 = (k + 1 >= 0 && k + 1 < det) ? to_float(row[k + 1]) : 0.f;
     const float d = t1 - t0;
     S[idx] = make_float2(ABS ? fmaf(-(float)(k - det / 2), d, t0) : t0, d);
 }
 
-template <bool ABS>
-__global__ void k_relayout_sino2d(const float *__restrict__ sino, int det, int nangles,
+template <bool ABS, class T>
+__global__ void k_relayout_sino2d(const T *__restrict__ sino, int det, int nangles,
                                   float2 *__restrict__ S) {
     wait_previous();
     relayout_sino2d_elem<ABS>(sino, det, nangles, S,
@@ -1482,9 +1483,9 @@ __global__ void __launch_bounds__(256, MINB)
 // through L1, the pair's absolute-position form is taken on the fly in the
 // re-layout's operations, and the groups' sums are added in order, so the
 // results are those of the staged tiles bit for bit.
-template <int G>
+template <int G, class T>
 __global__ void __launch_bounds__(32 * G)
-    k_bwd2d_direct(float *__restrict__ vol, const float *__restrict__ sino,
+    k_bwd2d_direct(float *__restrict__ vol, const T *__restrict__ sino,
                    const float4 *__restrict__ proj, int W, int H, int det, int nangles, float sx,
                    float sy, float ox, float oy, float ds, int per) {
     wait_previous();
@@ -1509,7 +1510,7 @@ __global__ void __launch_bounds__(32 * G)
             sB[group][lane] = proj[nangles + v0 + lane];
         }
         __syncwarp();
-        const float *row = sino + (size_t)v0 * det;
+        const T *row = sino + (size_t)v0 * det;
 #pragma unroll 1
         for (int j = 0; j < nv; ++j, row += det) {
             const float4 a = sA[group][j], b = sB[group][j];
@@ -1523,10 +1524,10 @@ __global__ void __launch_bounds__(32 * G)
             const float2 t = __fadd2_rd(ub, M2);
             const int k0 = (int)(__float_as_uint(t.x) - 0x4B400000u) + cq;
             const int k1 = (int)(__float_as_uint(t.y) - 0x4B400000u) + cq;
-            const float s00 = (unsigned)k0 < (unsigned)det ? __ldg(row + k0) : 0.f;
-            const float s01 = (unsigned)(k0 + 1) < (unsigned)det ? __ldg(row + k0 + 1) : 0.f;
-            const float s10 = (unsigned)k1 < (unsigned)det ? __ldg(row + k1) : 0.f;
-            const float s11 = (unsigned)(k1 + 1) < (unsigned)det ? __ldg(row + k1 + 1) : 0.f;
+            const float s00 = (unsigned)k0 < (unsigned)det ? to_float(__ldg(row + k0)) : 0.f;
+            const float s01 = (unsigned)(k0 + 1) < (unsigned)det ? to_float(__ldg(row + k0 + 1)) : 0.f;
+            const float s10 = (unsigned)k1 < (unsigned)det ? to_float(__ldg(row + k1)) : 0.f;
+            const float s11 = (unsigned)(k1 + 1) < (unsigned)det ? to_float(__ldg(row + k1 + 1)) : 0.f;
             const float d0 = s01 - s00, d1 = s11 - s10;
             const float g0 = fmaf(-(float)(k0 - cq), d0, s00), g1 = fmaf(-(float)(k1 - cq), d1, s10);
             const float2 v = make_float2(fmaf(ub.x, d0, g0), fmaf(ub.y, d1, g1));
@@ -1776,14 +1777,19 @@ int launch_plan2d_tables(Plan2d &p, cudaStream_t s) {
     return CG_OK;
 }
 
-int launch_relayout2d(const Plan2d &p, const float *vol, cudaStream_t s) {
+int launch_relayout2d(const Plan2d &p, const void *vol, bool half, cudaStream_t s) {
     dim3 grid(ceil_div(p.W + 2 * kPad, kTile), ceil_div(p.H + 2 * kPad, kTile));
     // the chunked forward's absolute-position shapes read the ABS form
     const bool abs_form = (p.algo_fwd == 4 || p.algo_fwd == 5) && cslab_abs(p.fwd_chunk_rows);
-    auto kernel = abs_form ? k_relayout2d<true> : k_relayout2d<false>;
-    CG_TRY(launch_after(kernel, grid, dim3(32, 8), 0, s, 1, vol, p.W, p.H, p.d_layA, p.d_layB,
-                        p.pitchA(), p.pitchB()));
-    return CG_OK;
+    auto launch = [&](auto kernel, auto *from) {
+        return launch_after(kernel, grid, dim3(32, 8), 0, s, 1, from, p.W, p.H, p.d_layA, p.d_layB,
+                            p.pitchA(), p.pitchB());
+    };
+    if (half)
+        return launch(abs_form ? k_relayout2d<true, __half> : k_relayout2d<false, __half>,
+                      static_cast<const __half *>(vol));
+    return launch(abs_form ? k_relayout2d<true, float> : k_relayout2d<false, float>,
+                  static_cast<const float *>(vol));
 }
 
 int launch_forward2d(const Plan2d &p, float *sino, cudaStream_t s) {
@@ -1804,14 +1810,19 @@ int launch_forward2d(const Plan2d &p, float *sino, cudaStream_t s) {
     return CG_OK;
 }
 
-int launch_relayout_sino2d(const Plan2d &p, const float *sino, cudaStream_t s) {
+int launch_relayout_sino2d(const Plan2d &p, const void *sino, bool half, cudaStream_t s) {
     const long long n = (long long)p.pitchS() * p.nangles;
     // the staged backprojector's absolute-position shapes read the ABS form
     const bool abs_form = (p.algo_bwd == 2 || p.algo_bwd == 3) && bwd_abs(p.bwd_min_blocks);
-    auto kernel = abs_form ? k_relayout_sino2d<true> : k_relayout_sino2d<false>;
-    CG_TRY(launch_after(kernel, ceil_div(n, 256), 256, 0, s, 1, sino, p.det, p.nangles,
-                        p.d_sinoP));
-    return CG_OK;
+    auto launch = [&](auto kernel, auto *from) {
+        return launch_after(kernel, ceil_div(n, 256), 256, 0, s, 1, from, p.det, p.nangles,
+                            p.d_sinoP);
+    };
+    if (half)
+        return launch(abs_form ? k_relayout_sino2d<true, __half> : k_relayout_sino2d<false, __half>,
+                      static_cast<const __half *>(sino));
+    return launch(abs_form ? k_relayout_sino2d<true, float> : k_relayout_sino2d<false, float>,
+                  static_cast<const float *>(sino));
 }
 
 // Streaming multiprocessors of the current device (looked up once per device).
@@ -1873,15 +1884,24 @@ int bwd_group_views(const Plan2d &p) {
     return best >= passes ? p.nangles : best * kSmViews;
 }
 
-int launch_backward2d_smem(const Plan2d &p, float *vol, const float *sino, cudaStream_t s) {
+int launch_backward2d_smem(const Plan2d &p, float *vol, const void *sino, bool half,
+                           cudaStream_t s) {
     const int per = bwd_group_views(p), groups = ceil_div(p.nangles, per);
     const bool standard = p.bwd_min_blocks == 68;
-    if (standard && bwd_direct(p))
-        return launch_after(groups > 4 ? k_bwd2d_direct<kDirectGroups> : k_bwd2d_direct<4>,
-                            dim3(ceil_div(p.W, 8), ceil_div(p.H, 8)), dim3(32, groups), 0, s, 1,
-                            vol, sino, p.d_bproj, p.W, p.H, p.det, p.nangles, p.sx, p.sy, p.ox,
-                            p.oy, p.ds, per);
-    if (int rc = launch_relayout_sino2d(p, sino, s)) return rc;
+    if (standard && bwd_direct(p)) {
+        auto direct = [&](auto kernel, auto *from) {
+            return launch_after(kernel, dim3(ceil_div(p.W, 8), ceil_div(p.H, 8)), dim3(32, groups),
+                                0, s, 1, vol, from, p.d_bproj, p.W, p.H, p.det, p.nangles, p.sx,
+                                p.sy, p.ox, p.oy, p.ds, per);
+        };
+        if (half)
+            return direct(groups > 4 ? k_bwd2d_direct<kDirectGroups, __half>
+                                     : k_bwd2d_direct<4, __half>,
+                          static_cast<const __half *>(sino));
+        return direct(groups > 4 ? k_bwd2d_direct<kDirectGroups, float> : k_bwd2d_direct<4, float>,
+                      static_cast<const float *>(sino));
+    }
+    if (int rc = launch_relayout_sino2d(p, sino, half, s)) return rc;
     if (p.bwd_sym != 0) {
         // the first quadrant's tiles, each with its three turned copies
         const int half = p.W / 2;

@@ -64,19 +64,21 @@ namespace {
 // of a small image (with launch_after, 64^2 x 360 views 10.2 -> 6.0 us a call in a
 // CUDA graph, 12.3 -> 6.3 outside one), and a batch moves all its volumes in one
 // launch.
-__device__ __forceinline__ void fill_tile(cudaSurfaceObject_t surf, const float *__restrict__ vol,
+template <class T>
+__device__ __forceinline__ void fill_tile(cudaSurfaceObject_t surf, const T *__restrict__ vol,
                                           int W, int H, int bx, int by) {
     const int x = bx * 32 + (threadIdx.x & 31);
     if (x >= W) return;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int y = by * 32 + 8 * i + (threadIdx.x >> 5);
-        if (y < H) surf2Dwrite(vol[(size_t)y * W + x], surf, x * (int)sizeof(float), y);
+        if (y < H) surf2Dwrite(to_float(vol[(size_t)y * W + x]), surf, x * (int)sizeof(float), y);
     }
 }
 
+template <class T>
 __global__ void __launch_bounds__(256)
-    k_fill_tex(cudaSurfaceObject_t surf, const float *__restrict__ vol, int W, int H) {
+    k_fill_tex(cudaSurfaceObject_t surf, const T *__restrict__ vol, int W, int H) {
     wait_previous();
     fill_tile(surf, vol, W, H, blockIdx.x, blockIdx.y);
 }
@@ -316,12 +318,16 @@ __global__ void __launch_bounds__(256)
 
 int tex_blocks(const Plan2d &p) { return ceil_div(p.det, kTexCells) * ceil_div(p.nangles, 8); }
 
-int launch_forward2d_tex(Plan2d &p, const float *vol, float *sino, cudaStream_t s) {
+int launch_forward2d_tex(Plan2d &p, const void *vol, bool half, float *sino, cudaStream_t s) {
     if (int rc = ensure_vol_texture(p)) return rc;
     const dim3 grid(ceil_div(p.det, kTexCells), ceil_div(p.nangles, 8));
     if (grid.y > 65535) return set_error(CG_ERR_INVALID, "too many views for one launch");
-    if (int rc = launch_after(k_fill_tex, dim3(ceil_div(p.W, 32), ceil_div(p.H, 32)), 256, 0, s, 1,
-                              p.surf_vol, vol, p.W, p.H))
+    auto fill = [&](auto kernel, auto *from) {
+        return launch_after(kernel, dim3(ceil_div(p.W, 32), ceil_div(p.H, 32)), 256, 0, s, 1,
+                            p.surf_vol, from, p.W, p.H);
+    };
+    if (int rc = half ? fill(k_fill_tex<__half>, static_cast<const __half *>(vol))
+                      : fill(k_fill_tex<float>, static_cast<const float *>(vol)))
         return rc;
     return launch_after(k_fwd2d_tex, grid, 256, 0, s, 1, p.tex_vol, sino, p.d_src, p.d_u0, p.d_du,
                         p.W, p.H, p.det, p.nangles, p.sx, p.sy);
