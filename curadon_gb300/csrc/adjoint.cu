@@ -239,11 +239,13 @@ __global__ void k_fold2d(float *__restrict__ vol, const float2 *__restrict__ A,
 // slice, up or down, within the same row and column, its near quad (the one
 // the ray meets first) is the held far one and both go out as one atomic.
 // Against merging upwards-going rays' slices only: 2446 -> 2116 us at 128^3 x
-// 180, 40.2 -> 33.1 ms at 256^3 x 360, 202 -> 177 us at 64^3 x 90; bound by
-// the L2's reductions as before (16 sectors per warp's atomic), of which a
-// sample now takes 1.4 instead of 1.7.  (Merging across lanes as well was
-// slower: 4.01 ms at 128^3 x 180 -- about 9 % of a warp's same-step targets
-// coincide.)
+// 180, 40.2 -> 33.1 ms at 256^3 x 360, 202 -> 177 us at 64^3 x 90; a sample now
+// takes 1.4 atomics instead of 1.7.  Bound by their way from the L1 to the L2
+// (81 %; 16 sectors per warp's atomic) and by issue (72 %): floors by FP32 adds
+// instead of conversions and 32-bit offsets (48 registers instead of 54, five
+// blocks per SM) then 2116 -> 2016 us, 177 -> 166.  (Merging across lanes as
+// well was slower: 4.01 ms at 128^3 x 180 -- about 9 % of a warp's same-step
+// targets coincide.)
 // The band-major block `lin`'s cell of this thread.
 __device__ __forceinline__ void adj3d_band_cell(int lin, int utiles, int P, int &iu, int &iv,
                                                 int &view) {
@@ -256,8 +258,11 @@ __device__ __forceinline__ void adj3d_band_cell(int lin, int utiles, int P, int 
     iv = band * 8 + (warp >> 2) * 4 + (lane >> 3);
 }
 
+__device__ __forceinline__ float2 times(float a, float2 b) { return make_float2(a * b.x, a * b.y); }
+__device__ __forceinline__ float2 plus(float2 a, float2 b) { return __fadd2_rn(a, b); }
+
 // One ray's scatter (the cell (iu, iv) of `view`).
-template <bool QUAD, bool MERGE>
+template <bool QUAD, bool MERGE, class Off = size_t>
 __device__ __forceinline__ void adj3d_ray(void *__restrict__ A, void *__restrict__ B,
                                           const float *__restrict__ sino,
                                           const float4 *__restrict__ torg,
@@ -303,15 +308,59 @@ __device__ __forceinline__ void adj3d_ray(void *__restrict__ A, void *__restrict
     void *L = xmajor ? B : A;
     const int Na = xmajor ? Z : X, Nc = xmajor ? X : Z;
     const int pa = Na + 2 * kPad, pb = Y + 2 * kPad;
+    float t = tmin;
+    if constexpr (QUAD && MERGE) {
+        // the held contributions, of the near slice (the one the ray enters a
+        // cell by) and the far one, and the near one's element; floors by adds
+        // rounded down (bits of p + 1.5 * 2^23 = floor(p) + const), indices past
+        // the padding clamped into it, where what lands is dropped
+        constexpr float kMagic = 12582912.0f;
+        constexpr unsigned base = 0x4B400000u - (unsigned)kPad;
+        const bool down = dc < 0.f;
+        const unsigned acap = (unsigned)(Na + kPad), bcap = (unsigned)(Y + kPad),
+                       ccap = (unsigned)(Nc + kPad);
+        const Off slice = (Off)pa * pb, ahead = down ? (Off)0 - slice : slice;
+        float4 *q = static_cast<float4 *>(L);
+        Off held_at = ~(Off)0;
+        float2 n0 = make_float2(0.f, 0.f), n1 = n0, f0 = n0, f1 = n0;  // rows b, b + 1
+        for (int k = 0; k <= nsteps + 1; ++k) {
+            if (!(t <= tmax)) break;
+            const float xa = fmaf(da, t, sa), xb = fmaf(dy, t, s.y), xc = fmaf(dc, t, sc);
+            const float ta = __fadd_rd(xa, kMagic), tb = __fadd_rd(xb, kMagic),
+                        tc = __fadd_rd(xc, kMagic);
+            const float wa = __fadd_rn(xa, -__fadd_rn(ta, -kMagic));
+            const float wb = __fadd_rn(xb, -__fadd_rn(tb, -kMagic));
+            const float wc = __fadd_rn(xc, -__fadd_rn(tc, -kMagic));
+            const unsigned ia = min(__float_as_uint(ta) - base, acap);
+            const unsigned ib = min(__float_as_uint(tb) - base, bcap);
+            const unsigned ic = min(__float_as_uint(tc) - base, ccap);
+            const Off at = ((Off)(ic + (down ? 1u : 0u)) * pb + ib) * pa + ia;
+            const float vc = 1.f - wc, wn = down ? wc : vc, wf = down ? vc : wc;
+            const float c0 = c * (1.f - wb), c1 = c * wb;
+            const float2 w = make_float2(1.f - wa, wa);
+            const float2 m0 = times(c0 * wn, w), m1 = times(c1 * wn, w);
+            const float2 g0 = times(c0 * wf, w), g1 = times(c1 * wf, w);
+            if (at == held_at) {  // the same cell again
+                n0 = plus(n0, m0), n1 = plus(n1, m1), f0 = plus(f0, g0), f1 = plus(f1, g1);
+            } else {
+                const bool held = held_at != ~(Off)0, next = at == held_at + ahead;
+                if (held) atomicAdd(q + held_at, make_float4(n0.x, n0.y, n1.x, n1.y));
+                if (held && !next)
+                    atomicAdd(q + (Off)(held_at + ahead), make_float4(f0.x, f0.y, f1.x, f1.y));
+                n0 = m0, n1 = m1;
+                if (next) n0 = plus(n0, f0), n1 = plus(n1, f1);
+                f0 = g0, f1 = g1, held_at = at;
+            }
+            t = march_next(t, k, tmin, h, exact_t);
+        }
+        if (held_at != ~(Off)0) {
+            atomicAdd(q + held_at, make_float4(n0.x, n0.y, n1.x, n1.y));
+            atomicAdd(q + (Off)(held_at + ahead), make_float4(f0.x, f0.y, f1.x, f1.y));
+        }
+        return;
+    }
     const float amax = (float)Na, bmax = (float)Y, cmax = (float)Nc;
     const float lo = -(float)kPad;
-    float t = tmin;
-    // MERGE: the held contributions, of the near slice (the one the ray enters
-    // a cell by) and the far one, and the near one's element
-    const bool down = dc < 0.f;
-    const int slice = pa * pb, ahead = down ? -slice : slice;
-    size_t held_at = ~(size_t)0;
-    float4 near = make_float4(0.f, 0.f, 0.f, 0.f), far = near;
     for (int k = 0; k <= nsteps + 1; ++k) {
         if (!(t <= tmax)) break;
         const float pa_ = fmaf(da, t, sa), pb_ = fmaf(dy, t, s.y), pc_ = fmaf(dc, t, sc);
@@ -322,24 +371,7 @@ __device__ __forceinline__ void adj3d_ray(void *__restrict__ A, void *__restrict
         const size_t i00 = ((size_t)((int)fc + kPad) * pb + ((int)fb + kPad)) * pa + ((int)fa + kPad);
         const float c00 = c * (1.f - wb) * (1.f - wc), c10 = c * wb * (1.f - wc);
         const float c01 = c * (1.f - wb) * wc, c11 = c * wb * wc;
-        if constexpr (QUAD && MERGE) {
-            float4 *q = static_cast<float4 *>(L);
-            const float4 lower = make_float4(c00 * (1.f - wa), c00 * wa, c10 * (1.f - wa), c10 * wa);
-            const float4 upper = make_float4(c01 * (1.f - wa), c01 * wa, c11 * (1.f - wa), c11 * wa);
-            const size_t at = down ? i00 + slice : i00;
-            const float4 n1 = down ? upper : lower, f1 = down ? lower : upper;
-            if (at == held_at) {  // the same cell again
-                near.x += n1.x, near.y += n1.y, near.z += n1.z, near.w += n1.w;
-                far.x += f1.x, far.y += f1.y, far.z += f1.z, far.w += f1.w;
-            } else {
-                const bool held = held_at != ~(size_t)0, next = at == held_at + ahead;
-                if (held) atomicAdd(q + held_at, near);
-                if (held && !next) atomicAdd(q + (held_at + ahead), far);
-                near = n1;
-                if (next) near.x += far.x, near.y += far.y, near.z += far.z, near.w += far.w;
-                far = f1, held_at = at;
-            }
-        } else if constexpr (QUAD) {
+        if constexpr (QUAD) {
             float4 *q = static_cast<float4 *>(L) + i00;
             atomicAdd(q, make_float4(c00 * (1.f - wa), c00 * wa, c10 * (1.f - wa), c10 * wa));
             atomicAdd(q + (size_t)pa * pb,
@@ -353,16 +385,9 @@ __device__ __forceinline__ void adj3d_ray(void *__restrict__ A, void *__restrict
         }
         t = march_next(t, k, tmin, h, exact_t);
     }
-    if constexpr (QUAD && MERGE) {
-        if (held_at != ~(size_t)0) {
-            float4 *q = static_cast<float4 *>(L) + held_at;
-            atomicAdd(q, near);
-            atomicAdd(q + ahead, far);
-        }
-    }
 }
 
-template <bool QUAD, bool BAND = false, bool MERGE = false>
+template <bool QUAD, bool BAND = false, bool MERGE = false, class Off = size_t>
 __global__ void __launch_bounds__(256)
     k_adj3d(void *__restrict__ A, void *__restrict__ B, const float *__restrict__ sino,
             const float4 *__restrict__ torg, const float4 *__restrict__ tdu,
@@ -377,7 +402,7 @@ __global__ void __launch_bounds__(256)
         iv = blockIdx.y * blockDim.y + threadIdx.y;
         view = blockIdx.z;
     }
-    adj3d_ray<QUAD, MERGE>(A, B, sino, torg, tdu, tdv, tsrc, X, Y, Z, U, V, exact_t, iu, iv, view);
+    adj3d_ray<QUAD, MERGE, Off>(A, B, sino, torg, tdu, tdv, tsrc, X, Y, Z, U, V, exact_t, iu, iv, view);
 }
 
 // vol[z][y][x] += A[z][y][x].x + A[z][y][x-1].y + B[x][y][z].x + B[x][y][z-1].y
@@ -443,8 +468,9 @@ __global__ void __launch_bounds__(256)
     const Prob3d &q = probs[i];
     int iu, iv, view;
     adj3d_band_cell(blockIdx.x - start[i], q.utiles, q.P, iu, iv, view);
-    adj3d_ray<true, true>(q.adjA, q.adjB, q.sino, q.forg, q.fdu, q.fdv, q.fsrc, q.X, q.Y, q.Z, q.U,
-                          q.V, q.exact_t != 0, iu, iv, view);
+    // (a batch's problems have fewer than 2^32 elements)
+    adj3d_ray<true, true, unsigned>(q.adjA, q.adjB, q.sino, q.forg, q.fdu, q.fdv, q.fsrc, q.X, q.Y,
+                                    q.Z, q.U, q.V, q.exact_t != 0, iu, iv, view);
 }
 
 __global__ void __launch_bounds__(256)
@@ -573,8 +599,12 @@ int launch_adjoint3d(Plan3d &p, float *vol, const float *sino, cudaStream_t s) {
         if (int rc = ensure_adj3d_quads(p)) return rc;
         CG_TRY_CUDA(cudaMemsetAsync(p.d_quadA, 0, elems * sizeof(float4), s));
         CG_TRY_CUDA(cudaMemsetAsync(p.d_quadB, 0, elems * sizeof(float4), s));
-        auto kq = p.adj_merge ? (band ? k_adj3d<true, true, true> : k_adj3d<true, false, true>)
-                              : (band ? k_adj3d<true, true> : k_adj3d<true, false>);
+        // (32-bit element offsets where they do)
+        const bool wide = elems >= (1ull << 32);
+        auto kq = !p.adj_merge ? (band ? k_adj3d<true, true> : k_adj3d<true, false>)
+                  : wide       ? (band ? k_adj3d<true, true, true> : k_adj3d<true, false, true>)
+                               : (band ? k_adj3d<true, true, true, unsigned>
+                                       : k_adj3d<true, false, true, unsigned>);
         CG_TRY(launch_after(kq, grid, dim3(32, 8), 0, s, 1, p.d_quadA, p.d_quadB, sino, p.d_forg,
                             p.d_fdu, p.d_fdv, p.d_fsrc, p.X, p.Y, p.Z, p.U, p.V, p.nangles, utiles,
                             p.exact_t));
