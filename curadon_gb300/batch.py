@@ -8,7 +8,7 @@ tensors.  ``forward()`` then projects every volume into its sinogram and
 The buffers stay bound, so both calls can be captured in a CUDA graph
 (``torch.cuda.graph``) and an iteration loop replayed without launch
 overhead.  The forward is the texture-unit ray march (``forward="texture"``,
-default: one array copy per problem, then one launch), the FP32 register
+default: a launch that fills every array, a launch), the FP32 register
 march (``forward="registers"``) or each problem's own plan default
 (``forward="plans"``: the chunked shared-memory forward for problems from
 704^2 pixels, in one re-layout and one bundle launch over all of them, the
