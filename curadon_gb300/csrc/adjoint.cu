@@ -512,8 +512,16 @@ int launch_batch2d_adjoint(const Prob2d *probs, const int *starts,
 int launch_adjoint2d(Plan2d &p, float *vol, const float *sino, cudaStream_t s) {
     const size_t na = adj2d_quad_elems(p, true);
     const size_t nb = adj2d_quad_elems(p, false);
-    dim3 block(p.fwd_bx, p.fwd_by);
-    dim3 grid(ceil_div(p.det, p.fwd_bx), ceil_div(p.nangles, p.fwd_by));
+    // small blocks: a block's slot is free again when its own rays end, and
+    // rays end far apart (the scatter keeps no more than their positions).  One
+    // warp where two of them wait for each of the SMs' 32 block slots, else two
+    // (blocks of 8 / 2 / 1 warps, us: 256^2 x 256 92 / 68 / 72, 513^2 x 437 374 /
+    // 343 / 329, 1024^2 x 1024 2675 / 2574 / 2541)
+    const long long warps = (long long)ceil_div(p.det, 32) * p.nangles;
+    int rows = warps >= 2LL * 32 * sm_count() ? 1 : 2;
+    while (rows < 8 && ceil_div(p.nangles, rows) > 65535) rows *= 2;
+    dim3 block(32, rows);
+    dim3 grid(ceil_div(p.det, 32), ceil_div(p.nangles, rows));
     if (grid.y > 65535) return set_error(CG_ERR_INVALID, "too many views for one launch");
     const dim3 fgrid(ceil_div(p.W, 32), ceil_div(p.H, 8));
     // quad accumulators up to 160 MB (2230^2), a little above what the L2 can
@@ -594,7 +602,12 @@ int launch_adjoint3d(Plan3d &p, float *vol, const float *sino, cudaStream_t s) {
     const bool quad = p.adj_quad != 0;
     const bool fits = 2 * elems * (quad ? sizeof(float4) : sizeof(float2)) <= (96u << 20);
     const bool band = (p.adj_band > 0 || (p.adj_band < 0 && !fits)) && bblocks < (1ll << 31);
-    dim3 grid = band ? dim3((unsigned)bblocks) : dim3(utiles, ceil_div(p.V, 8), p.nangles);
+    // view-major blocks of four warps (of eight / four, us: 128^3 x 180 2019 /
+    // 2001, 100^3 x 150 837 / 826, 64^3 x 90 166 / 160; two or one: the same)
+    const int rows = band || ceil_div(p.V, 4) > 65535 ? 8 : 4;
+    const dim3 grid = band ? dim3((unsigned)bblocks)
+                           : dim3(utiles, ceil_div(p.V, rows), p.nangles);
+    const dim3 block(32, rows);
     if (quad) {
         if (int rc = ensure_adj3d_quads(p)) return rc;
         CG_TRY_CUDA(cudaMemsetAsync(p.d_quadA, 0, elems * sizeof(float4), s));
@@ -605,7 +618,7 @@ int launch_adjoint3d(Plan3d &p, float *vol, const float *sino, cudaStream_t s) {
                   : wide       ? (band ? k_adj3d<true, true, true> : k_adj3d<true, false, true>)
                                : (band ? k_adj3d<true, true, true, unsigned>
                                        : k_adj3d<true, false, true, unsigned>);
-        CG_TRY(launch_after(kq, grid, dim3(32, 8), 0, s, 1, p.d_quadA, p.d_quadB, sino, p.d_forg,
+        CG_TRY(launch_after(kq, grid, block, 0, s, 1, p.d_quadA, p.d_quadB, sino, p.d_forg,
                             p.d_fdu, p.d_fdv, p.d_fsrc, p.X, p.Y, p.Z, p.U, p.V, p.nangles, utiles,
                             p.exact_t));
         CG_TRY(launch_after(k_fold3d_quad, ceil_div(n, 256), 256, 0, s, 1, vol, p.d_quadA,
@@ -615,7 +628,7 @@ int launch_adjoint3d(Plan3d &p, float *vol, const float *sino, cudaStream_t s) {
     CG_TRY_CUDA(cudaMemsetAsync(p.d_volA, 0, p.volA_elems * sizeof(float2), s));
     CG_TRY_CUDA(cudaMemsetAsync(p.d_volB, 0, p.volB_elems * sizeof(float2), s));
     auto kp = band ? k_adj3d<false, true> : k_adj3d<false, false>;
-    CG_TRY(launch_after(kp, grid, dim3(32, 8), 0, s, 1, p.d_volA, p.d_volB, sino, p.d_forg,
+    CG_TRY(launch_after(kp, grid, block, 0, s, 1, p.d_volA, p.d_volB, sino, p.d_forg,
                         p.d_fdu, p.d_fdv, p.d_fsrc, p.X, p.Y, p.Z, p.U, p.V, p.nangles, utiles,
                         p.exact_t));
     CG_TRY(launch_after(k_fold3d, ceil_div(n, 256), 256, 0, s, 1, vol, p.d_volA, p.d_volB, p.X,

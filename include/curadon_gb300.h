@@ -98,7 +98,7 @@ int cg_plan2d_destroy(cg_plan2d *plan);
 /* The reference's read-write `forward_block_x` / `forward_block_y`
   * (plan.cu:57-58, plan_2d.hpp:184-186): here they set the detector-cells x
  * views shape of one thread block (x a multiple of 32, x * y <= 256) of the
- * ray-by-ray register forward and of the matched adjoint. */
+ * ray-by-ray register forward. */
 int cg_plan2d_get_forward_block(const cg_plan2d *plan, uint64_t *bx, uint64_t *by);
 int cg_plan2d_set_forward_block(cg_plan2d *plan, uint64_t bx, uint64_t by);
 
