@@ -101,7 +101,7 @@ struct Plan2d {
     float *d_vol32 = nullptr, *d_sino32 = nullptr;
 
     // matched adjoint: quad accumulators (float4 per padded texel of layA /
-    // layB), allocated on first use; adj_quad -1 = when both fit in 96 MB,
+    // layB), allocated on first use; adj_quad -1 = when both fit in 160 MB,
     // 1 = always, 0 = never (pair accumulators in layA / layB)
     float4 *d_quadA = nullptr, *d_quadB = nullptr;
     int adj_quad = -1;
