@@ -458,10 +458,15 @@ class FanRays:
             t1, t2 = (-1 - src[k]) / d[k], (size[k] - src[k]) / d[k]
             lo = torch.minimum(torch.maximum(t1, lo), torch.maximum(t2, lo))
             hi = torch.maximum(torch.minimum(t1, hi), torch.minimum(t2, hi))
+        # a ray that misses, or only touches a corner (lo == hi), takes no steps;
+        # its positions are finite all the same, since they become indices
         hit = lo <= hi - 1e-6
-        m = torch.maximum((d[0] * (hi - lo)).abs(), (d[1] * (hi - lo)).abs())
-        self.steps = torch.where(hit, m.round(), torch.zeros_like(m)).reshape(-1)
-        self.v = [(d[k] * (hi - lo) / m).reshape(-1) for k in range(2)]
+        zero = torch.zeros_like(lo)
+        lo, length = torch.where(hit, lo, zero), torch.where(hit, hi - lo, zero)
+        m = torch.maximum((d[0] * length).abs(), (d[1] * length).abs())
+        self.steps = m.round().reshape(-1)
+        m = torch.where(hit, m, torch.ones_like(m))
+        self.v = [(d[k] * length / m).reshape(-1) for k in range(2)]
         self.p = [(src[k] + d[k] * lo).reshape(-1) - 0.5 for k in range(2)]
         self.norm = torch.hypot(*self.v)
         self.pitch = size[0] + 4
