@@ -2,6 +2,7 @@
 order, so their results are equal bit for bit -- at the edges of the bundles
 (64 / 128 cells, 4 / 8 views), where windows outgrow their buffers (few views
 over a full turn) and in batches."""
+import numpy as np
 import pytest
 import torch
 
@@ -51,3 +52,22 @@ def test_batched_bundles_agree(cuda_device, monkeypatch):
     torch.cuda.synchronize()
     for s, e in zip(sinos, expect):
         assert torch.equal(s, e)
+
+
+@pytest.mark.parametrize("n,angle", [(6000, 2.0), (8192, 2.0), (16384, 0.4)])
+def test_bundles_of_wide_images_agree(cuda_device, monkeypatch, n, angle):
+    """Both bundles' windows hold the samples whose columns, running sums, have
+    strayed from their rays' lines, and those that strayed off the padding."""
+    g = fan_config(n, 8, 3 * n // 2)
+    g["angles"] = (angle + 0.0007 * np.arange(8)).astype(np.float32)
+    gen = torch.Generator(device=cuda_device).manual_seed(n)
+    vol = torch.rand((n, n), device=cuda_device, generator=gen)
+    out = []
+    for bundle in ("small", "large"):
+        monkeypatch.setenv("CURADON_GB300_ALGO", f"fwd2d_bundle={bundle}")
+        geom = FanGeometry(**g)
+        assert geom.plan.algorithm[0] == "chunked"
+        monkeypatch.delenv("CURADON_GB300_ALGO")
+        out.append(forward(vol, torch.full(geom.sinogram_shape(), -1.0, device=cuda_device), geom))
+    torch.cuda.synchronize()
+    assert torch.equal(*out)

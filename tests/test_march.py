@@ -45,3 +45,23 @@ def test_bundled_register_forward(cuda_device, monkeypatch, name, geom):
     torch.cuda.synchronize()
     assert torch.equal(alone, rays)
     assert torch.equal(batched, rays)
+
+
+@pytest.mark.parametrize("n", [6000, 8192, 16384])
+def test_bundled_register_forward_of_wide_images(cuda_device, monkeypatch, n):
+    """A ray's column is a running sum, which at these sizes strays from its line
+    by a column and more: the bundle's windows hold those samples too."""
+    g = fan_config(n, 8, 3 * n // 2)
+    g["angles"] = (0.0007 * np.arange(8)).astype(np.float32)  # windows within their buffers
+    geom = FanGeometry(**g)
+    gen = torch.Generator(device=cuda_device).manual_seed(n)
+    vol = torch.rand((n, n), device=cuda_device, generator=gen)
+    alone = torch.full(geom.sinogram_shape(), -1.0, device=cuda_device)
+    rays = torch.full_like(alone, -3.0)
+    forward(vol, alone, geom, exact=True)
+    monkeypatch.setenv("CURADON_GB300_ALGO", "fwd2d=alu,fwd2d_march=off")
+    plan = geom._make_plan()
+    monkeypatch.delenv("CURADON_GB300_ALGO")
+    forward_2d(vol, rays, plan)
+    torch.cuda.synchronize()
+    assert torch.equal(alone, rays)
