@@ -527,14 +527,22 @@ int launch_adjoint2d(Plan2d &p, float *vol, const float *sino, cudaStream_t s) {
     // quad accumulators up to 160 MB (2230^2), a little above what the L2 can
     // hold: quads / pairs, us: 1448^2 x 1024 5235 / 6695, 2048^2 x 360 3842 /
     // 4864, 3000^2 x 360 10698 / 10162, 4096^2 x 180 15771 / 11110.  A plan
-    // that gets no room for them (or is first used under capture, where nothing
-    // may be allocated) scatters into pairs, which every plan has
+    // that gets no room for them scatters into pairs, which every plan has, from
+    // then on; one first used under capture, where nothing may be allocated,
+    // until it is used outside
     bool quad = p.adj_quad > 0;
     if (p.adj_quad < 0 && (na + nb) * sizeof(float4) <= (160u << 20)) {
         cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
         if (!p.d_quadA) CG_TRY_CUDA(cudaStreamIsCapturing(s, &capture));
-        quad = capture == cudaStreamCaptureStatusNone && ensure_adj2d_quads(p) == CG_OK;
-        if (!quad) clear_error();
+        if (capture == cudaStreamCaptureStatusNone) {
+            const int rc = ensure_adj2d_quads(p);
+            if (rc && rc != CG_ERR_NOMEM) return rc;
+            quad = rc == CG_OK;
+            if (!quad) {
+                clear_error();
+                p.adj_quad = 0;
+            }
+        }
     }
     if (quad) {
         if (int rc = ensure_adj2d_quads(p)) return rc;
@@ -562,7 +570,6 @@ int ensure_adj3d_quads(Plan3d &p) {
     const size_t elems = (size_t)(p.X + 2 * kPad) * (p.Y + 2 * kPad) * (p.Z + 2 * kPad);
     CG_TRY_CUDA(cudaMalloc(&p.d_quadA, elems * sizeof(float4)));
     if (cudaMalloc(&p.d_quadB, elems * sizeof(float4)) != cudaSuccess) {
-        (void)cudaGetLastError();
         cudaFree(p.d_quadA);
         p.d_quadA = nullptr;
         return set_error(CG_ERR_NOMEM, "no room for the matched adjoint's accumulators");

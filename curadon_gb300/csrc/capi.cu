@@ -20,6 +20,9 @@ thread_local std::string g_last_error;
 
 int set_error(int code, const std::string &msg) {
     g_last_error = msg;
+    // a CUDA call's failure is reported here and not again by the next launch's
+    // check (the runtime keeps the last one until it is read)
+    if (code == CG_ERR_CUDA || code == CG_ERR_NOMEM) (void)cudaGetLastError();
     return code;
 }
 

@@ -10,6 +10,7 @@ import numpy as np
 import pytest
 import torch
 
+from conftest import rel_l2
 from curadon_gb300 import ConeGeometry, FanGeometry, adjoint, forward
 from curadon_gb300.phantom import cone_config, fan_config
 
@@ -55,3 +56,49 @@ def test_3d(cuda_device, monkeypatch, order, shape, nangles, det):
     g = cone_config(max(shape), nangles, det)
     g.update(vol_shape=shape)
     check(ConeGeometry(**g), shape, cuda_device)
+
+
+def test_adjoint_2d_when_memory_is_short(cuda_device):
+    """A plan without room for the quad accumulators (2 x 67 MB) scatters into
+    pairs, for good, and leaves no error behind for the next plan."""
+    geom, ref = (FanGeometry(**fan_config(2048, 6)) for _ in range(2))
+    y = torch.rand(geom.sinogram_shape(), device=cuda_device)
+    expect, out = (torch.zeros((2048, 2048), device=cuda_device) for _ in range(2))
+    adjoint(y, expect, ref)
+    geom.exact_plan
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    free, _ = torch.cuda.mem_get_info()
+    filler = torch.empty(max(0, free - (24 << 20)), dtype=torch.uint8, device=cuda_device)
+    try:
+        adjoint(y, out, geom)
+        torch.cuda.synchronize()
+    finally:
+        del filler
+        torch.cuda.empty_cache()
+    other = FanGeometry(**fan_config(64, 6))  # its creation checks its launch
+    small = torch.ones((64, 64), device=cuda_device)
+    forward(small, torch.zeros(other.sinogram_shape(), device=cuda_device), other)
+    assert rel_l2(out.cpu(), expect.cpu()) < 1e-5
+    torch.cuda.synchronize()
+    free, _ = torch.cuda.mem_get_info()
+    adjoint(y, out, geom)
+    torch.cuda.synchronize()
+    assert torch.cuda.mem_get_info()[0] > free - (64 << 20)
+    assert rel_l2(out.cpu(), 2 * expect.cpu()) < 1e-5
+
+
+def test_adjoint_2d_first_used_under_capture(cuda_device):
+    geom, ref = (FanGeometry(**fan_config(300, 90)) for _ in range(2))
+    y = torch.rand(geom.sinogram_shape(), device=cuda_device)
+    expect, out = (torch.zeros((300, 300), device=cuda_device) for _ in range(2))
+    adjoint(y, expect, ref)
+    geom.exact_plan
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        adjoint(y, out, geom)
+    graph.replay()
+    adjoint(y, out, geom)  # outside: with its quads
+    graph.replay()
+    torch.cuda.synchronize()
+    assert rel_l2(out.cpu(), 3 * expect.cpu()) < 1e-5
