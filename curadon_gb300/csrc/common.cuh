@@ -359,7 +359,7 @@ int launch_backward2d_smem(const Plan2d &p, float *vol, const void *sino, bool h
                            cudaStream_t s);
 // blocks of the quarter-turn backprojection of a W x W image
 int sym_quadrant_blocks(int W);
-// views whose sum the staged backprojection adds to the volume at a time
+// views that the staged backprojection sums at a time (the groups' sums follow)
 int bwd_group_views(const Plan2d &p);
 int sm_count();
 // rows: the chunked forward's compiled shape (kFwdChunkShapes: 443, 474, 484)

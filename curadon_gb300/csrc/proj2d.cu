@@ -917,10 +917,11 @@ __device__ __forceinline__ void add_cluster_parts(float *part, int count, int gr
     for (int run = (tid >> 5) * groups + group; run < count / 32; run += warps * groups) {
         float *to = at(run * 32 + lane);
         if (!to) continue;
-        float v = *to;
+        const float before = *to;
+        float v = 0.f;
         for (int g = 0; g < groups; ++g)
             v = fmaf(*cluster.map_shared_rank(part + run * 32 + lane, g), inv, v);
-        *to = v;
+        *to = before + v;
     }
     cluster.sync();  // the parts stay until every CTA has read them
 }
@@ -957,13 +958,14 @@ constexpr int kSmWin = 128;   // pairs of one view's row staged for a tile
 // R: pixels per thread (rows 8 apart), so tiles of 32 x 8R pixels; every
 // pixel's sum runs over the views in the same order whatever R, so results
 // do not depend on it.
-// A pixel's views are summed in groups of `per` views (bwd_group_views): each
-// group's sum is added to the volume, one group after the other.  CLUSTER:
-// the CTAs of a cluster take one group each (`group`) and add their parts in
-// that order through distributed shared memory; otherwise the block takes the
-// groups in turn.  The results are the same bits.
+// A pixel's views are summed in groups of `per` views (bwd_group_views), the
+// groups' sums one after the other, and their sum is added to the volume (once:
+// a value there that is large beside it is rounded once).  GROUPS = 2: the CTAs
+// of a cluster take one group each (`group`) and add their parts in that order
+// through distributed shared memory; 1: the block takes the groups in turn, the
+// same bits; 0: one group.
 template <bool PK, bool MAGIC = false, int VU = 2, bool CPA = false, bool ABS = false,
-          bool MAPQ = false, bool BULK = false, int R = kSmRows, bool CLUSTER = false>
+          bool MAPQ = false, bool BULK = false, int R = kSmRows, int GROUPS = 0>
 __device__ __forceinline__ void bwd2d_smem_tile(float *__restrict__ vol,
                                                 const float2 *__restrict__ S,
                                                 const float4 *__restrict__ proj, int W, int H,
@@ -1014,17 +1016,16 @@ __device__ __forceinline__ void bwd2d_smem_tile(float *__restrict__ vol,
             mbar_fence_init();
         }
     }
-    // adds the group's sums to the volume and starts the next group
-    auto flush = [&]() {
-        if (x >= W) return;
+    // GROUPS = 1: the sum of the groups before; takes the present one's in.  (In
+    // shared memory: in registers, which the samples need, a batch of twelve
+    // backprojections took 753 us, with the sums added to the volume each time
+    // 744, so 739.)
+    __shared__ float total[GROUPS == 1 ? R : 1][GROUPS == 1 ? 256 : 1];
+    auto next_group = [&](bool first) {
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-            const int y = y0 + 8 * r;
             float &a = (r & 1) ? acc2[r >> 1].y : acc2[r >> 1].x;
-            if (y < H) {
-                float &v = vol[(size_t)y * W + x];
-                v = fmaf(a, inv, v);
-            }
+            total[r][tid] = fmaf(a, inv, first ? 0.f : total[r][tid]);
             a = 0.f;
         }
     };
@@ -1034,13 +1035,13 @@ __device__ __forceinline__ void bwd2d_smem_tile(float *__restrict__ vol,
     // has not seen complete.  The tile's results are then not to be trusted
     // and the give-up is counted for cg_wait_timeouts.
     int gave_up = 0;
-    const int va = CLUSTER ? group * per : 0;
-    const int vb = CLUSTER ? min(va + per, nangles) : nangles;
+    const int va = GROUPS == 2 ? group * per : 0;
+    const int vb = GROUPS == 2 ? min(va + per, nangles) : nangles;
     int vgroup = va + per;  // end of the group being summed
     for (int v0 = va; v0 < vb; v0 += kSmViews) {
         const int nv = min(kSmViews, vb - v0);
-        if (!CLUSTER && v0 == vgroup) {
-            flush();
+        if (GROUPS == 1 && v0 == vgroup) {
+            next_group(vgroup == per);
             vgroup += per;
         }
         if constexpr (BULK) {
@@ -1218,7 +1219,7 @@ __device__ __forceinline__ void bwd2d_smem_tile(float *__restrict__ vol,
             if (gave_up) mbar_wait(bar, phase, kWaitTries);
         }
     }
-    if constexpr (CLUSTER) {
+    if constexpr (GROUPS == 2) {
         // the parts lie in the CTAs' staged rows, which are no longer read
         static_assert(sizeof(srow) >= sizeof(float) * 256 * R, "parts fit the staged rows");
         float *part = reinterpret_cast<float *>(srow);
@@ -1233,7 +1234,17 @@ __device__ __forceinline__ void bwd2d_smem_tile(float *__restrict__ vol,
             return px < W && py < H ? vol + (size_t)py * W + px : nullptr;
         });
     } else {
-        flush();
+        const bool groups = GROUPS == 1 && per < nangles;
+        if (groups) next_group(false);
+        if (x >= W) return;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int y = y0 + 8 * r;
+            if (y >= H) continue;
+            float &v = vol[(size_t)y * W + x];
+            const float a = (r & 1) ? acc2[r >> 1].y : acc2[r >> 1].x;
+            v = groups ? v + total[r][tid] : fmaf(a, inv, v);
+        }
     }
 }
 
@@ -1502,9 +1513,9 @@ __global__ void __launch_bounds__(256, MINB)
                  const float4 *__restrict__ proj, int W, int H, int det, int nangles, float sx,
                  float sy, float ox, float oy, float ds, int per) {
     wait_previous();
-    bwd2d_smem_tile<PK, MAGIC, VU, CPA, ABS, MAPQ, BULK, R>(vol, S, proj, W, H, det, nangles,
-                                                            sx, sy, ox, oy, ds, blockIdx.x,
-                                                            blockIdx.y, per);
+    // (the bulk variant has its groups in clusters, k_bwd2d_cluster)
+    bwd2d_smem_tile<PK, MAGIC, VU, CPA, ABS, MAPQ, BULK, R, BULK ? 0 : 1>(
+        vol, S, proj, W, H, det, nangles, sx, sy, ox, oy, ds, blockIdx.x, blockIdx.y, per);
 }
 
 // Small images: no staging and no re-layout.  Each warp takes 8 x 8 pixels
@@ -1570,9 +1581,10 @@ __global__ void __launch_bounds__(32 * G)
     for (int e = group * 32 + lane; e < 64; e += groups * 32) {
         const int px = blockIdx.x * 8 + (e & 7), py = blockIdx.y * 8 + (e >> 3);
         if (px >= W || py >= H) continue;
-        float v = vol[(size_t)py * W + px];
+        const float before = vol[(size_t)py * W + px];
+        float v = 0.f;
         for (int g = 0; g < groups; ++g) v = fmaf(part[g][e], inv, v);
-        vol[(size_t)py * W + px] = v;
+        vol[(size_t)py * W + px] = before + v;
     }
 }
 
@@ -1583,7 +1595,7 @@ __global__ void __launch_bounds__(256, MINB)
                     const float4 *__restrict__ proj, int W, int H, int det, int nangles, float sx,
                     float sy, float ox, float oy, float ds, int per) {
     wait_previous();
-    bwd2d_smem_tile<true, true, 4, true, true, true, true, kSmRows, true>(
+    bwd2d_smem_tile<true, true, 4, true, true, true, true, kSmRows, 2>(
         vol, S, proj, W, H, det, nangles, sx, sy, ox, oy, ds, blockIdx.x, blockIdx.y, per,
         blockIdx.z);
 }
@@ -1682,10 +1694,9 @@ __global__ void __launch_bounds__(256, 4)
     const Prob2d &q = probs[i];
     const int local = blockIdx.x - start[i];
     const int gx = (q.W + 31) / 32;
-    bwd2d_smem_tile<true, true, 4, true, true, true, true>(q.vol, q.sinoP, q.bproj, q.W, q.H,
-                                                           q.det, q.nangles, q.sx, q.sy, q.ox,
-                                                           q.oy, q.ds, local % gx, local / gx,
-                                                           q.bwd_per);
+    bwd2d_smem_tile<true, true, 4, true, true, true, true, kSmRows, 1>(
+        q.vol, q.sinoP, q.bproj, q.W, q.H, q.det, q.nangles, q.sx, q.sy, q.ox, q.oy, q.ds,
+        local % gx, local / gx, q.bwd_per);
 }
 
 // The quarter-turn symmetric tile of the single-problem default for the

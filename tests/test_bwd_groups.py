@@ -49,3 +49,24 @@ def test_split_views_nonfinite(cuda_device, n, views):
     torch.cuda.synchronize()
     assert torch.equal(torch.isnan(alone), torch.isnan(batched))
     assert torch.equal(torch.nan_to_num(alone), torch.nan_to_num(batched))
+
+
+@pytest.mark.parametrize("n,views", [(64, 360), (120, 700), (300, 400), (640, 640), (900, 450)])
+def test_a_large_volume_is_rounded_once(cuda_device, n, views):
+    """However many groups a pixel's views are summed in, a value that the volume
+    holds already takes one rounding of the result (2^-24 of it) and one of the
+    backprojection itself."""
+    geom = FanGeometry(**fan_config(n, views))
+    gen = torch.Generator(device=cuda_device).manual_seed(n)
+    y = torch.rand(geom.sinogram_shape(), device=cuda_device, generator=gen)
+    start = 1e6 + torch.rand((n, n), device=cuda_device, generator=gen)
+    plain = torch.zeros_like(start)
+    backward(y, plain, geom)
+    alone, batched = start.clone(), start.clone()
+    backward(y, alone, geom)
+    Batch2d([geom], [batched], [y]).backward()
+    torch.cuda.synchronize()
+    exact = start.double() + plain.double()
+    bound = 2.0 ** -24 * (1.0001 * exact.abs() + plain.double().abs())
+    for out in (alone, batched):
+        assert bool(((out.double() - exact).abs() <= bound).all())
