@@ -516,11 +516,12 @@ int launch_fft(const float *in, float *out, const float *h, const float *pre, in
     return CG_OK;
 }
 
-// Rows that are filtered by FFT: from 160 cells (direct / FFT, us in a CUDA
-// graph, rows x cells: 90 x 128 9.1 / 9.3, 128 x 182 11.9 / 10.2, 256 x 363 22
-// / 12) to 4096, whose tables and spectrum still fit a block.  Fewer than 48
-// rows keep the direct sum, whose two kernels agree bit for bit.
-bool fft_rows(int N, int nrows) { return nrows >= 48 && N >= 160 && N <= 4096; }
+// Rows that are filtered by FFT: from 160 cells to 4096, whose tables and
+// spectrum still fit a block; however many rows, so that a row's result is the
+// same alone and in a stack.  Direct / FFT, us in a CUDA graph: 90 rows of 128
+// cells 9.1 / 9.3; one row of 160 10.1 / 8.7, of 256 15.2 / 9.6, of 1449 92 /
+// 13.3, of 4096 268 / 18.3; 47 rows 10.8 / 9.2, 15.6 / 9.6, 95 / 13.3, 272 / 18.7.
+bool fft_rows(int N) { return N >= 160 && N <= 4096; }
 
 }  // namespace
 
@@ -534,7 +535,7 @@ int launch_filter_rows(const float *in, float *out, const float *h, const float 
     // ramp-like taps of long rows by FFT; the direct kernel launched after it
     // returns at once for them and does the others (the taps are known on the
     // device only)
-    const bool fft = fft_rows(N, nrows);
+    const bool fft = fft_rows(N);
     if (fft) {
         const int rc = N <= 512    ? launch_fft<512>(in, out, h, pre, nrows, N, scale, s)
                        : N <= 1024 ? launch_fft<1024>(in, out, h, pre, nrows, N, scale, s)
