@@ -134,6 +134,9 @@ class plan_2d:
 
     @property
     def forward_block_x(self) -> int:
+        """Detector cells of a thread block of the ray-by-ray register forward
+        (``cg_plan2d_set_forward_block``); the other forwards and the adjoint
+        have tiles of their own, and no result depends on it."""
         return self._block()[0]
 
     @forward_block_x.setter
@@ -142,6 +145,7 @@ class plan_2d:
 
     @property
     def forward_block_y(self) -> int:
+        """Views of such a block."""
         return self._block()[1]
 
     @forward_block_y.setter

@@ -96,9 +96,11 @@ int cg_plan2d_create_vec(cg_plan2d **plan, int device, uint32_t vol_prec,
 int cg_plan2d_destroy(cg_plan2d *plan);
 
 /* The reference's read-write `forward_block_x` / `forward_block_y`
-  * (plan.cu:57-58, plan_2d.hpp:184-186): here they set the detector-cells x
- * views shape of one thread block (x a multiple of 32, x * y <= 256) of the
- * ray-by-ray register forward. */
+ * (plan.cu:57-58, plan_2d.hpp:184-186): the detector-cells x views shape of one
+ * thread block (x a multiple of 32, x * y <= 256) of the ray-by-ray register
+ * forward.  The other forwards and the matched adjoint have tiles of their own,
+ * and the register forward normally runs in bundles, so the pair is kept, checked
+ * and returned but changes no launch of theirs; results never depend on it. */
 int cg_plan2d_get_forward_block(const cg_plan2d *plan, uint64_t *bx, uint64_t *by);
 int cg_plan2d_set_forward_block(cg_plan2d *plan, uint64_t bx, uint64_t by);
 
@@ -283,12 +285,12 @@ int cg_filter_rows(const float *in, float *out, const float *h, const float *pre
 
 /* A batch binds `count` float32 2D plans (any sizes and geometries, each
  * plan at most once) to their device volumes and sinograms.  Each direction
-  * of the whole batch then runs as two to four launches over (problem, tile)
- * work lists instead of two launches per problem: the serving / many-problem entry
- * point, capturable in a CUDA graph because the buffers are bound.  The
+ * of the whole batch then runs as two to four launches over (problem, tile)
+ * work lists instead of two launches per problem: the serving / many-problem
+ * entry point, capturable in a CUDA graph because the buffers are bound.  The
  * batched forward is the texture-unit ray march (algorithm 1, default: one
- * launch fills every problem's array, one traces its rays) or the register ray march
- * (algorithm 0: a re-layout launch and one launch), the batched
+ * launch fills every problem's array, one traces its rays) or the register
+ * ray march (algorithm 0: a re-layout launch and one launch), the batched
  * backprojection the staged one (algorithm 2); results equal cg_forward_2d /
  * cg_backward_2d with those algorithms bit for bit.  A batch must not run
  * concurrently with other calls on its plans.  No counterpart call in the

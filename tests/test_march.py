@@ -65,3 +65,18 @@ def test_bundled_register_forward_of_wide_images(cuda_device, monkeypatch, n):
     forward_2d(vol, rays, plan)
     torch.cuda.synchronize()
     assert torch.equal(alone, rays)
+
+
+def test_forward_block_shapes_the_ray_by_ray_kernel(cuda_device, monkeypatch):
+    g = FanGeometry(**fan_config(100, 37, 211))
+    vol = torch.rand((100, 100), device=cuda_device)
+    expect = forward(vol, torch.zeros(g.sinogram_shape(), device=cuda_device), g, exact=True)
+    monkeypatch.setenv("CURADON_GB300_ALGO", "fwd2d=alu,fwd2d_march=off")
+    plan = g._make_plan()
+    for bx, by in ((32, 8), (64, 2), (256, 1), (32, 1)):
+        plan.forward_block_y = 1
+        plan.forward_block_x, plan.forward_block_y = bx, by
+        assert (plan.forward_block_x, plan.forward_block_y) == (bx, by)
+        out = torch.full_like(expect, -1.0)
+        forward_2d(vol, out, plan)
+        assert torch.equal(out, expect)
