@@ -26,9 +26,9 @@ namespace {
 // A sample's far row is the next one's near row, so while the ray stays in its
 // column the contributions are held in registers: a quad goes out complete
 // every second sample (pairs: every sample).  Bound by the L2's reductions:
-// per call 413 -> 366 us at 513^2 x 437, 3057 -> 2672 at 1024^2 x 1024, 103 ->
-// 92 at 256^2 x 256; pairs 5991 -> 4852 at 2048^2 x 360, 4422 -> 3530 at
-// 1024^2 x 1024.
+// this took a call from 413 to 366 us at 513^2 x 437, 3057 to 2672 at 1024^2 x
+// 1024, 103 to 92 at 256^2 x 256 (with the launch's small blocks 329, 2541 and 68
+// now); pairs 5991 to 4852 at 2048^2 x 360, 4422 to 3530 at 1024^2 x 1024.
 template <bool QUAD>
 __device__ __forceinline__ void adj2d_ray(void *__restrict__ accA, void *__restrict__ accB,
                                           const float *__restrict__ sino,
@@ -402,7 +402,8 @@ __global__ void __launch_bounds__(256)
         iv = blockIdx.y * blockDim.y + threadIdx.y;
         view = blockIdx.z;
     }
-    adj3d_ray<QUAD, MERGE, Off>(A, B, sino, torg, tdu, tdv, tsrc, X, Y, Z, U, V, exact_t, iu, iv, view);
+    adj3d_ray<QUAD, MERGE, Off>(A, B, sino, torg, tdu, tdv, tsrc, X, Y, Z, U, V, exact_t, iu,
+                                iv, view);
 }
 
 // vol[z][y][x] += A[z][y][x].x + A[z][y][x-1].y + B[x][y][z].x + B[x][y][z-1].y

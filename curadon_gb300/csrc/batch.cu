@@ -180,7 +180,6 @@ int cg_batch2d_create(cg_batch2d **batch, cg_plan2d *const *plans, float *const 
         if (int rc = ensure_vol_texture(*plans[i])) return rc;
         q.tex = p.tex_vol, q.surf = p.surf_vol;
         q.quadA = p.d_quadA, q.quadB = p.d_quadB;
-        q.chunked = batch_chunked(p) ? 1 : 0;
         q.bwd_sym = p.bwd_sym;
         q.bwd_per = bwd_group_views(p);
         int blocks[kBatchStages];

@@ -75,20 +75,24 @@ bool listed(const int (&list)[N], int v) {
 
 // Overrides of a new plan's algorithms for measurement and testing, read
 // from CURADON_GB300_ALGO: comma-separated key=value tokens, e.g.
-// "fwd2d=tex,bwd2d_minb=48".  Keys: fwd2d = alu | tex | cslab |
-// cslab<443 | 474 | 484>; fwd2d_bundle = small | large (the chunked forward's
-// bundles); fwd2d_march = off (the register forward ray by ray); bwd2d = alu | tex | smem; bwd2d_minb = 27 | 48 | 68
-// (staged backprojector variants); adj2d = pair | quad; fwd3d = alu | tex3 |
-// quad | mixed; fwd3d_tex = 0..8 (texture warps of 8 in the mixed forward);
-// fwd3d_unroll = 1 | 2 (the mixed forward's texture fetches one or three at a time);
-// fwd3d_block = BXxBYxBZ; bwd3d = quad | pair (general kernel on row-pair
-// quads or on 8-byte pairs, its fallback where quads do not fit) | ax8m5
-// (axial runs);
-// adj3d = pair | quad; adj3d_order = band | view; adj3d_merge = 0 | 1;
-// (adj3d_agg, once atomics merged across lanes, is ignored);
-// t3d = step | exact (running-sum or drift-free sample parameters of the 3D
-// ray marches).  Unknown tokens are ignored; without the variable every plan
-// starts at the measured defaults.
+// "fwd2d=tex,bwd2d_minb=48".  Keys:
+//   fwd2d = alu | tex | cslab | cslab<443 | 474 | 484>
+//   fwd2d_bundle = small | large (the chunked forward's bundles)
+//   fwd2d_march = off (the register forward ray by ray)
+//   bwd2d = alu | tex | smem; bwd2d_sym = off | on (quarter turns)
+//   bwd2d_minb = 27 | 48 | 68 (staged backprojector variants)
+//   adj2d = pair | quad
+//   fwd3d = alu | tex3 | quad | mixed
+//   fwd3d_tex = 0..8 (texture warps of 8 in the mixed forward)
+//   fwd3d_unroll = 1 | 2 (its texture fetches one or three at a time)
+//   fwd3d_block = BXxBYxBZ (the 3D texture forward)
+//   bwd3d = quad | pair (general kernel on row-pair quads or on 8-byte pairs, its
+//     fallback where quads do not fit) | ax8m5 (axial runs)
+//   adj3d = pair | quad; adj3d_order = band | view; adj3d_merge = 0 | 1
+//   t3d = step | exact (running-sum or drift-free sample parameters of the 3D
+//     ray marches)
+// Unknown tokens are ignored; without the variable every plan starts at the
+// measured defaults.
 void apply_algo_env(Plan2d *p2, Plan3d *p3) {
     const char *env = std::getenv("CURADON_GB300_ALGO");
     if (!env) return;

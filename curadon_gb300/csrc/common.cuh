@@ -165,7 +165,6 @@ struct Prob2d {
     cudaTextureObject_t tex;   // the plan's volume texture (texture forward)
     cudaSurfaceObject_t surf;  // and its array for writing
     float4 *quadA, *quadB;    // matched adjoint: the plan's quad accumulators
-    int chunked;              // the batched "plans" forward runs the chunked kernel
     int bwd_sym;              // the plan's quarter-turn symmetry (Plan2d::bwd_sym)
     int bwd_per;              // views summed at a time (bwd_group_views)
 };
@@ -323,7 +322,8 @@ struct SideStream {
 
 int launch_relayout_sino2d(const Plan2d &p, const void *sino, bool half, cudaStream_t s);
 // batches (proj2d.cu): blocks of each stage of one problem, and the launch of
-// one direction over a batch whose starts hold 4 x (count + 1) block starts
+// one direction over a batch whose starts hold kBatchStages x (count + 1) block
+// starts
 void batch_blocks(const Plan2d &p, int blocks[kBatchStages]);
 // true where the batched "plans" forward runs the plan's chunked shape
 bool batch_chunked(const Plan2d &p);

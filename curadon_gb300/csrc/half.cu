@@ -72,15 +72,18 @@ int ensure_half_scratch(Plan2d &p, bool vol, bool sino) {
 }
 
 int widen_half(const void *in, float *out, long long n, cudaStream_t s) {
-    return launch_after(k_half_to_float, grid_for(n), 256, 0, s, 1, static_cast<const __half *>(in), out, n);
+    return launch_after(k_half_to_float, grid_for(n), 256, 0, s, 1,
+                        static_cast<const __half *>(in), out, n);
 }
 
 int narrow_to_half(const float *in, void *out, long long n, cudaStream_t s) {
-    return launch_after(k_float_to_half, grid_for(n), 256, 0, s, 1, in, static_cast<__half *>(out), n);
+    return launch_after(k_float_to_half, grid_for(n), 256, 0, s, 1, in,
+                        static_cast<__half *>(out), n);
 }
 
 int add_into_half(void *vol, const float *add, long long n, cudaStream_t s) {
-    return launch_after(k_add_to_half, grid_for(n), 256, 0, s, 1, static_cast<__half *>(vol), add, n);
+    return launch_after(k_add_to_half, grid_for(n), 256, 0, s, 1, static_cast<__half *>(vol),
+                        add, n);
 }
 
 }  // namespace cg

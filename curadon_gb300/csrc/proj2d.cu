@@ -632,39 +632,39 @@ __device__ __forceinline__ void cslab_bundle(const float2 *__restrict__ layA,
             auto samples = [&](auto down) {
                 auto at = [&](int k) { return decltype(down)::value ? K - 1 - k : k; };
 #pragma unroll
-            for (int g = 0; g < GV; ++g) {
-                const int rel = r0 - rlo[g];
-                if (rel >= 0 && rel + K <= len[g]) {
-                    // REUSE: row k's lower pair is row k-1's upper pair when the
-                    // column did not change (|step| <= 1 column per row), so
-                    // only the lanes whose column moved load it
-                    unsigned c_prev = 0xffffffffu;
-                    float2 hi_prev = make_float2(0.f, 0.f);
+                for (int g = 0; g < GV; ++g) {
+                    const int rel = r0 - rlo[g];
+                    if (rel >= 0 && rel + K <= len[g]) {
+                        // REUSE: row k's lower pair is row k-1's upper pair when the
+                        // column did not change (|step| <= 1 column per row), so
+                        // only the lanes whose column moved load it
+                        unsigned c_prev = 0xffffffffu;
+                        float2 hi_prev = make_float2(0.f, 0.f);
 #pragma unroll
-                    for (int k = 0; k < K; ++k) {
-                        float fp;
-                        const unsigned c = cs_column<ABS>(p[g], c0 - ic, cmax, fp);
-                        const float2 hi = b0[(at(k) + 1) * S + c];
-                        float2 lo;
-                        if (REUSE && c == c_prev) lo = hi_prev;
-                        else lo = b0[at(k) * S + c];
-                        acc[g].add(fp, lo, hi);
-                        if (REUSE) c_prev = c, hi_prev = hi;
-                        p[g] += V[g];
-                    }
-                } else {
-#pragma unroll
-                    for (int k = 0; k < K; ++k) {
-                        if ((unsigned)(rel + k) < (unsigned)len[g]) {
+                        for (int k = 0; k < K; ++k) {
                             float fp;
                             const unsigned c = cs_column<ABS>(p[g], c0 - ic, cmax, fp);
-                            const float2 lo = b0[at(k) * S + c], hi = b0[(at(k) + 1) * S + c];
+                            const float2 hi = b0[(at(k) + 1) * S + c];
+                            float2 lo;
+                            if (REUSE && c == c_prev) lo = hi_prev;
+                            else lo = b0[at(k) * S + c];
                             acc[g].add(fp, lo, hi);
+                            if (REUSE) c_prev = c, hi_prev = hi;
                             p[g] += V[g];
+                        }
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < K; ++k) {
+                            if ((unsigned)(rel + k) < (unsigned)len[g]) {
+                                float fp;
+                                const unsigned c = cs_column<ABS>(p[g], c0 - ic, cmax, fp);
+                                const float2 lo = b0[at(k) * S + c], hi = b0[(at(k) + 1) * S + c];
+                                acc[g].add(fp, lo, hi);
+                                p[g] += V[g];
+                            }
                         }
                     }
                 }
-            }
             };
             if (MARCH && desc) samples(std::true_type{});
             else samples(std::false_type{});
@@ -688,7 +688,8 @@ __device__ __forceinline__ void cslab_bundle(const float2 *__restrict__ layA,
                         // rows past the ray's last are loaded from it and dropped
                         const unsigned c = cs_column<ABS>(p[g], -kPad - ic, gcap, fp[k]);
                         const int m = min(rg + k, rb - 1);
-                        const float2 *rowp = lay + (size_t)((MARCH && desc ? -m : m) + kPad) * pitch + c;
+                        const int row = (MARCH && desc ? -m : m) + kPad;
+                        const float2 *rowp = lay + (size_t)row * pitch + c;
                         lo[k] = __ldg(rowp), hi[k] = __ldg(rowp + pitch);
                         if (rg + k < rb) p[g] += V[g];
                     }
@@ -704,7 +705,8 @@ __device__ __forceinline__ void cslab_bundle(const float2 *__restrict__ layA,
         if (__syncthreads_or(gave_up) && threadIdx.x == 0) {
             atomicAdd(&g_wait_timeouts, 1ull);
             for (int b = 0; b < 2; ++b)
-                if ((pending >> b) & 1u) mbar_wait(bar0 + 8u * (unsigned)b, (phases >> b) & 1u, kWaitTries);
+                if ((pending >> b) & 1u)
+                    mbar_wait(bar0 + 8u * (unsigned)b, (phases >> b) & 1u, kWaitTries);
         }
     }
 
@@ -1954,7 +1956,8 @@ int launch_backward2d_smem(const Plan2d &p, float *vol, const void *sino, bool h
     // two blocks takes 32 x 16-pixel tiles (two pixels per thread) instead,
     // four times the blocks, the same sums (unless clusters fill the SMs)
     const bool cluster = standard && groups > 1;
-    const bool small = !cluster && (long long)ceil_div(p.W, 32) * ceil_div(p.H, 8 * kSmRows) < 2LL * sm_count();
+    const long long tiles = (long long)ceil_div(p.W, 32) * ceil_div(p.H, 8 * kSmRows);
+    const bool small = !cluster && tiles < 2LL * sm_count();
     auto tile = [&](auto kernel) {
         const unsigned z = cluster ? groups : 1;
         return launch_after(kernel,

@@ -335,7 +335,8 @@ int launch_forward2d_tex(Plan2d &p, const void *vol, bool half, float *sino, cud
 
 int ensure_vol_texture(Plan2d &p) {
     int rc = CG_OK;
-    if (!p.arr_vol && (rc = alloc_array(&p.arr_vol, p.W, p.H, 0, cudaArraySurfaceLoadStore))) return rc;
+    if (!p.arr_vol && (rc = alloc_array(&p.arr_vol, p.W, p.H, 0, cudaArraySurfaceLoadStore)))
+        return rc;
     if (!p.surf_vol) {
         cudaResourceDesc res;
         std::memset(&res, 0, sizeof(res));
