@@ -18,6 +18,23 @@
 namespace cg {
 namespace {
 
+// Adds to two or four floats of global memory and returns nothing.  (Written
+// out: where the compiler does not see that a pointer is to global memory, as
+// with the accumulators of a batch's work list, atomicAdd may fetch the old
+// values as well: a batch of four 512^2 x 300 1240 us instead of 945.)
+__device__ __forceinline__ void red_add(float2 *p, float2 v) {
+    asm volatile("red.relaxed.gpu.global.add.v2.f32 [%0], {%1, %2};"
+                 :
+                 : "l"(__cvta_generic_to_global(p)), "f"(v.x), "f"(v.y)
+                 : "memory");
+}
+__device__ __forceinline__ void red_add(float4 *p, float4 v) {
+    asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};"
+                 :
+                 : "l"(__cvta_generic_to_global(p)), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
+                 : "memory");
+}
+
 // ------------------------------------------------------------ 2D
 
 // QUAD: one float4 per (row, column) of the layout holding the contributions
@@ -91,7 +108,7 @@ __device__ __forceinline__ void adj2d_ray(void *__restrict__ accA, void *__restr
         bool half = false;
         int held = 0;
         auto put = [&] {
-            atomicAdd(at, up ? make_float4(near.x, near.y, far.x, far.y)
+            red_add(at, up ? make_float4(near.x, near.y, far.x, far.y)
                              : make_float4(far.x, far.y, near.x, near.y));
         };
         for (int j = 0; j < n; ++j) {
@@ -123,15 +140,15 @@ __device__ __forceinline__ void adj2d_ray(void *__restrict__ accA, void *__restr
             const float fp = p - pf;
             const int ip = (int)pf;
             if (ip != at) {
-                if (j > 0) atomicAdd(row + at, held);
+                if (j > 0) red_add(row + at, held);
                 held = make_float2(0.f, 0.f), at = ip;
             }
-            atomicAdd(row + ip, make_float2(fmaf(cn, 1.f - fp, held.x), fmaf(cn, fp, held.y)));
+            red_add(row + ip, make_float2(fmaf(cn, 1.f - fp, held.x), fmaf(cn, fp, held.y)));
             held = make_float2(cf * (1.f - fp), cf * fp);
             p += vp;
             row += rstep;
         }
-        if (n > 0) atomicAdd(row + at, held);
+        if (n > 0) red_add(row + at, held);
     }
 }
 
@@ -344,9 +361,9 @@ __device__ __forceinline__ void adj3d_ray(void *__restrict__ A, void *__restrict
                 n0 = plus(n0, m0), n1 = plus(n1, m1), f0 = plus(f0, g0), f1 = plus(f1, g1);
             } else {
                 const bool held = held_at != ~(Off)0, next = at == held_at + ahead;
-                if (held) atomicAdd(q + held_at, make_float4(n0.x, n0.y, n1.x, n1.y));
+                if (held) red_add(q + held_at, make_float4(n0.x, n0.y, n1.x, n1.y));
                 if (held && !next)
-                    atomicAdd(q + (Off)(held_at + ahead), make_float4(f0.x, f0.y, f1.x, f1.y));
+                    red_add(q + (Off)(held_at + ahead), make_float4(f0.x, f0.y, f1.x, f1.y));
                 n0 = m0, n1 = m1;
                 if (next) n0 = plus(n0, f0), n1 = plus(n1, f1);
                 f0 = g0, f1 = g1, held_at = at;
@@ -354,8 +371,8 @@ __device__ __forceinline__ void adj3d_ray(void *__restrict__ A, void *__restrict
             t = march_next(t, k, tmin, h, exact_t);
         }
         if (held_at != ~(Off)0) {
-            atomicAdd(q + held_at, make_float4(n0.x, n0.y, n1.x, n1.y));
-            atomicAdd(q + (Off)(held_at + ahead), make_float4(f0.x, f0.y, f1.x, f1.y));
+            red_add(q + held_at, make_float4(n0.x, n0.y, n1.x, n1.y));
+            red_add(q + (Off)(held_at + ahead), make_float4(f0.x, f0.y, f1.x, f1.y));
         }
         return;
     }
@@ -373,15 +390,15 @@ __device__ __forceinline__ void adj3d_ray(void *__restrict__ A, void *__restrict
         const float c01 = c * (1.f - wb) * wc, c11 = c * wb * wc;
         if constexpr (QUAD) {
             float4 *q = static_cast<float4 *>(L) + i00;
-            atomicAdd(q, make_float4(c00 * (1.f - wa), c00 * wa, c10 * (1.f - wa), c10 * wa));
-            atomicAdd(q + (size_t)pa * pb,
+            red_add(q, make_float4(c00 * (1.f - wa), c00 * wa, c10 * (1.f - wa), c10 * wa));
+            red_add(q + (size_t)pa * pb,
                       make_float4(c01 * (1.f - wa), c01 * wa, c11 * (1.f - wa), c11 * wa));
         } else {
             float2 *p00 = static_cast<float2 *>(L) + i00;
-            atomicAdd(p00, make_float2(c00 * (1.f - wa), c00 * wa));
-            atomicAdd(p00 + pa, make_float2(c10 * (1.f - wa), c10 * wa));
-            atomicAdd(p00 + (size_t)pa * pb, make_float2(c01 * (1.f - wa), c01 * wa));
-            atomicAdd(p00 + (size_t)pa * pb + pa, make_float2(c11 * (1.f - wa), c11 * wa));
+            red_add(p00, make_float2(c00 * (1.f - wa), c00 * wa));
+            red_add(p00 + pa, make_float2(c10 * (1.f - wa), c10 * wa));
+            red_add(p00 + (size_t)pa * pb, make_float2(c01 * (1.f - wa), c01 * wa));
+            red_add(p00 + (size_t)pa * pb + pa, make_float2(c11 * (1.f - wa), c11 * wa));
         }
         t = march_next(t, k, tmin, h, exact_t);
     }
