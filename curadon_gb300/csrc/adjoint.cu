@@ -46,7 +46,10 @@ __device__ __forceinline__ void red_add(float4 *p, float4 v) {
 // this took a call from 413 to 366 us at 513^2 x 437, 3057 to 2672 at 1024^2 x
 // 1024, 103 to 92 at 256^2 x 256 (with the launch's small blocks 329, 2541 and 68
 // now); pairs 5991 to 4852 at 2048^2 x 360, 4422 to 3530 at 1024^2 x 1024.
-template <bool QUAD>
+// MERGE = false: every sample goes out by itself.  A ray is then a chain half as
+// long (a merged step, whose lanes part, takes 100 ns, a plain one 55), which
+// counts where the rays are too few for the L2 to matter.
+template <bool QUAD, bool MERGE>
 __device__ __forceinline__ void adj2d_ray(void *__restrict__ accA, void *__restrict__ accB,
                                           const float *__restrict__ sino,
                                           const float2 *__restrict__ tsrc,
@@ -96,6 +99,25 @@ __device__ __forceinline__ void adj2d_ray(void *__restrict__ accA, void *__restr
     long long ri = (long long)(iq + kPad) * pitch + kPad;  // element of the row start
     const long long rstep = (long long)sq * pitch;
     const float clo = c * (1.f - fq), chi = c * fq;
+    if constexpr (!MERGE) {
+        for (int j = 0; j < n; ++j) {
+            const float pf = fminf(fmaxf(floorf(p), -(float)kPad), pmax);
+            const float fp = p - pf;
+            const int ip = (int)pf;
+            // forward: lo = x + fp (y - x) -> weights (1 - fp, fp) on the pair
+            if constexpr (QUAD) {
+                red_add(static_cast<float4 *>(acc) + ri + ip,
+                        make_float4(clo * (1.f - fp), clo * fp, chi * (1.f - fp), chi * fp));
+            } else {
+                float2 *row = static_cast<float2 *>(acc) + ri;
+                red_add(row + ip, make_float2(clo * (1.f - fp), clo * fp));
+                red_add(row + pitch + ip, make_float2(chi * (1.f - fp), chi * fp));
+            }
+            p += vp;
+            ri += rstep;
+        }
+        return;
+    }
     // the near row of a sample is the far row of the one before
     const bool up = sq > 0;
     const float cn = up ? clo : chi, cf = up ? chi : clo;
@@ -152,15 +174,16 @@ __device__ __forceinline__ void adj2d_ray(void *__restrict__ accA, void *__restr
     }
 }
 
-template <bool QUAD>
+template <bool QUAD, bool MERGE>
 __global__ void __launch_bounds__(256)
     k_adj2d(void *__restrict__ accA, void *__restrict__ accB, const float *__restrict__ sino,
             const float2 *__restrict__ tsrc, const float2 *__restrict__ tu0,
             const float2 *__restrict__ tdu, int W, int H, int det, int nangles, float sx,
             float sy, int pa, int pb) {
     wait_previous();
-    adj2d_ray<QUAD>(accA, accB, sino, tsrc, tu0, tdu, W, H, det, nangles, sx, sy, pa, pb,
-                    blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y * blockDim.y + threadIdx.y);
+    adj2d_ray<QUAD, MERGE>(accA, accB, sino, tsrc, tu0, tdu, W, H, det, nangles, sx, sy, pa, pb,
+                           blockIdx.x * blockDim.x + threadIdx.x,
+                           blockIdx.y * blockDim.y + threadIdx.y);
 }
 
 // vol[y][x] += the four quad entries covering (x, y) in each layout.
@@ -205,6 +228,7 @@ __global__ void __launch_bounds__(256)
     }
 }
 
+template <bool MERGE>
 __global__ void __launch_bounds__(256)
     k_batch_adj2d(const Prob2d *__restrict__ probs, const int *__restrict__ start, int count) {
     wait_previous();
@@ -212,9 +236,9 @@ __global__ void __launch_bounds__(256)
     const Prob2d &q = probs[i];
     const int local = blockIdx.x - start[i];
     const int gx = (q.det + 31) / 32;
-    adj2d_ray<true>(q.quadA, q.quadB, q.sino, q.src, q.u0, q.du, q.W, q.H, q.det, q.nangles, q.sx,
-                    q.sy, q.pa, q.pb, (local % gx) * 32 + threadIdx.x,
-                    (local / gx) * 8 + threadIdx.y);
+    adj2d_ray<true, MERGE>(q.quadA, q.quadB, q.sino, q.src, q.u0, q.du, q.W, q.H, q.det,
+                           q.nangles, q.sx, q.sy, q.pa, q.pb, (local % gx) * 32 + threadIdx.x,
+                           (local / gx) * 8 + threadIdx.y);
 }
 
 __global__ void __launch_bounds__(256)
@@ -515,12 +539,24 @@ int ensure_adj2d_quads(Plan2d &p) {
     return CG_OK;
 }
 
+// Whether that many warps of rays hold their contributions (adj2d_ray's MERGE):
+// from six (pairs: four) for every SM.  Below, plain / merged, us: 256^2 x 1
+// view (12 warps) 19 / 31, 512^2 x 16 (368) 41 / 55, 2048^2 x 6 (546) 197 / 236,
+// 256^2 x 64 (768) 33 / 35; above, 2048^2 x 12 (1092) 290 / 272, 512^2 x 64 (1472)
+// 77 / 74, 1024^2 x 96 (4416) 361 / 323; pairs 3000^2 x 4 (532) 254 / 291, 2300^2 x 6
+// (612) 270 / 228.
+static bool adj2d_merges(long long warps, bool quad) {
+    return warps >= (quad ? 6LL : 4LL) * sm_count();
+}
+
 int launch_batch2d_adjoint(const Prob2d *probs, const int *starts,
                            const int totals[kBatchStages], int count, cudaStream_t s) {
     const dim3 tile(32, 8);
     CG_TRY(launch_after(k_batch_adj2d_zero, totals[4], 256, 0, s, 1, probs,
                         starts + 4 * (count + 1), count));
-    CG_TRY(launch_after(k_batch_adj2d, totals[5], tile, 0, s, 1, probs, starts + 5 * (count + 1),
+    const auto scatter = adj2d_merges(8LL * totals[5], true) ? k_batch_adj2d<true>
+                                                             : k_batch_adj2d<false>;
+    CG_TRY(launch_after(scatter, totals[5], tile, 0, s, 1, probs, starts + 5 * (count + 1),
                         count));
     CG_TRY(launch_after(k_batch_fold2d, totals[6], tile, 0, s, 1, probs, starts + 6 * (count + 1),
                         count));
@@ -544,12 +580,16 @@ int launch_adjoint2d(Plan2d &p, float *vol, const float *sino, cudaStream_t s) {
     const dim3 fgrid(ceil_div(p.W, 32), ceil_div(p.H, 8));
     // quad accumulators up to 160 MB (2230^2), a little above what the L2 can
     // hold: quads / pairs, us: 1448^2 x 1024 5235 / 6695, 2048^2 x 360 3842 /
-    // 4864, 3000^2 x 360 10698 / 10162, 4096^2 x 180 15771 / 11110.  A plan
+    // 4864, 3000^2 x 360 10698 / 10162, 4096^2 x 180 15771 / 11110; from 96 MB on
+    // for 24 warps of rays and more for every SM, since clearing and folding them
+    // takes 40 us longer (2048^2 x 1 view 135 / 97, x 12 271 / 236, x 31 531 / 522,
+    // x 48 740 / 766).  A plan
     // that gets no room for them scatters into pairs, which every plan has, from
     // then on; one first used under capture, where nothing may be allocated,
     // until it is used outside
     bool quad = p.adj_quad > 0;
-    if (p.adj_quad < 0 && (na + nb) * sizeof(float4) <= (160u << 20)) {
+    const size_t most = warps >= 24LL * sm_count() ? 160u << 20 : 96u << 20;
+    if (p.adj_quad < 0 && (na + nb) * sizeof(float4) <= most) {
         cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
         if (!p.d_quadA) CG_TRY_CUDA(cudaStreamIsCapturing(s, &capture));
         if (capture == cudaStreamCaptureStatusNone) {
@@ -562,11 +602,13 @@ int launch_adjoint2d(Plan2d &p, float *vol, const float *sino, cudaStream_t s) {
             }
         }
     }
+    const bool merge = adj2d_merges(warps, quad);
     if (quad) {
         if (int rc = ensure_adj2d_quads(p)) return rc;
         CG_TRY_CUDA(cudaMemsetAsync(p.d_quadA, 0, na * sizeof(float4), s));
         CG_TRY_CUDA(cudaMemsetAsync(p.d_quadB, 0, nb * sizeof(float4), s));
-        CG_TRY(launch_after(k_adj2d<true>, grid, block, 0, s, 1, p.d_quadA, p.d_quadB, sino,
+        const auto scatter = merge ? k_adj2d<true, true> : k_adj2d<true, false>;
+        CG_TRY(launch_after(scatter, grid, block, 0, s, 1, p.d_quadA, p.d_quadB, sino,
                             p.d_src, p.d_u0, p.d_du, p.W, p.H, p.det, p.nangles, p.sx, p.sy,
                             p.pitchA(), p.pitchB()));
         CG_TRY(launch_after(k_fold2d_quad, fgrid, dim3(32, 8), 0, s, 1, vol, p.d_quadA, p.d_quadB,
@@ -575,7 +617,8 @@ int launch_adjoint2d(Plan2d &p, float *vol, const float *sino, cudaStream_t s) {
     }
     CG_TRY_CUDA(cudaMemsetAsync(p.d_layA, 0, na * sizeof(float2), s));
     CG_TRY_CUDA(cudaMemsetAsync(p.d_layB, 0, nb * sizeof(float2), s));
-    CG_TRY(launch_after(k_adj2d<false>, grid, block, 0, s, 1, p.d_layA, p.d_layB, sino, p.d_src,
+    const auto scatter = merge ? k_adj2d<false, true> : k_adj2d<false, false>;
+    CG_TRY(launch_after(scatter, grid, block, 0, s, 1, p.d_layA, p.d_layB, sino, p.d_src,
                         p.d_u0, p.d_du, p.W, p.H, p.det, p.nangles, p.sx, p.sy, p.pitchA(),
                         p.pitchB()));
     CG_TRY(launch_after(k_fold2d, fgrid, dim3(32, 8), 0, s, 1, vol, p.d_layA, p.d_layB, p.W, p.H,

@@ -12,6 +12,7 @@ import torch
 
 from conftest import rel_l2
 from curadon_gb300 import ConeGeometry, FanGeometry, adjoint, forward
+from curadon_gb300.batch import Batch2d
 from curadon_gb300.phantom import cone_config, fan_config
 
 pytestmark = pytest.mark.gpu
@@ -61,7 +62,7 @@ def test_3d(cuda_device, monkeypatch, order, shape, nangles, det):
 def test_adjoint_2d_when_memory_is_short(cuda_device):
     """A plan without room for the quad accumulators (2 x 67 MB) scatters into
     pairs, for good, and leaves no error behind for the next plan."""
-    geom, ref = (FanGeometry(**fan_config(2048, 6)) for _ in range(2))
+    geom, ref = (FanGeometry(**fan_config(2048, 64)) for _ in range(2))
     y = torch.rand(geom.sinogram_shape(), device=cuda_device)
     expect, out = (torch.zeros((2048, 2048), device=cuda_device) for _ in range(2))
     adjoint(y, expect, ref)
@@ -102,3 +103,23 @@ def test_adjoint_2d_first_used_under_capture(cuda_device):
     graph.replay()
     torch.cuda.synchronize()
     assert rel_l2(out.cpu(), 3 * expect.cpu()) < 1e-5
+
+
+@pytest.mark.parametrize("n,views", [(7, 1), (40, 1), (300, 1), (300, 77), (300, 78), (1300, 1),
+                                     (1300, 2), (1800, 8), (1800, 9), (2300, 5), (2300, 6)])
+def test_adjoint_2d_of_few_rays(cuda_device, n, views):
+    """Few rays scatter sample by sample, more hold their contributions: the
+    transpose of the exact forward on both sides of the lines, alone and in a
+    batch (on 152 SMs: 912 warps of rays for quads, 608 for pairs)."""
+    geom = FanGeometry(**fan_config(n, views))
+    gen = torch.Generator(cuda_device).manual_seed(n + views)
+    x = torch.rand((n, n), device=cuda_device, generator=gen)
+    y = torch.rand(geom.sinogram_shape(), device=cuda_device, generator=gen)
+    ax, aty, batched = torch.zeros_like(y), torch.zeros_like(x), torch.zeros_like(x)
+    forward(x, ax, geom, exact=True)
+    adjoint(y, aty, geom)
+    Batch2d([geom], [batched], [y], forward="registers").adjoint()
+    torch.cuda.synchronize()
+    lhs = float((ax.double() * y.double()).sum())
+    for out in (aty, batched):
+        assert abs(lhs - float((x.double() * out.double()).sum())) < 1e-5 * abs(lhs)
