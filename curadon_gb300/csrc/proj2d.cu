@@ -777,11 +777,23 @@ __global__ void __launch_bounds__(128, 5)
                  blockIdx.y, blockIdx.z);
 }
 
-// Its window table packs columns in 16 bits, its grid 4 views per row.
+// Its window table packs columns in 16 bits, its grid 4 views per row.  Rays of
+// less than 256 samples do not pay for a bundle's set-up once there are more
+// bundles than nine for every SM, nor do the shortest at all.  Ray by ray / this,
+// us: 32^2 x 8 views 10.2 / 14.5, 64^2 x 90 25.1 / 18.6, x 720 (720 bundles) 23.6 /
+// 24.0, x 1440 24.2 / 37.1, 128^2 x 720 (1080) 41.6 / 37.6, x 1440 (2160) 53.4 /
+// 66.4, 200^2 x 360 (900) 66.7 / 45.6, x 720 (1800) 60.2 / 67.8, 256^2 x 720 (2160)
+// 95 / 88, x 1440 149 / 141.
 static bool marches(const Plan2d &p) {
+    const long long bundles = 2LL * ceil_div(p.det, 64) * ceil_div(p.nangles, 4);
+    const int side = std::max(p.W, p.H);
     return p.fwd_march && std::max(p.pitchA(), p.pitchB()) < 32768 &&
-           ceil_div(p.nangles, 4) <= 65535;
+           ceil_div(p.nangles, 4) <= 65535 &&
+           (side >= 256 || (side >= 64 && bundles <= 9LL * sm_count()));
 }
+// In a batch, small images have company: their bundles are many (64 of 64^2 x 30
+// views 45 us ray by ray, 63 so; 16 of 96^2 x 90 51, 62).
+static bool batch_marches(const Plan2d &p) { return marches(p) && std::max(p.W, p.H) >= 256; }
 
 static size_t cslab_smem(int stride) { return 2 * sizeof(float2) * (kCsRows + 1) * stride; }
 
@@ -1738,10 +1750,10 @@ void batch_blocks(const Plan2d &p, int blocks[kBatchStages]) {
     blocks[7] = chunked ? blocks[0] : 0;
     blocks[8] = chunked ? ceil_div(p.det, 128) * ceil_div(p.nangles, 8) * 2 : 0;
     blocks[9] = chunked ? 0 : blocks[1];
-    blocks[11] = marches(p) ? ceil_div(p.det, 64) * ceil_div(p.nangles, 4) * 2 : 0;
+    blocks[11] = batch_marches(p) ? ceil_div(p.det, 64) * ceil_div(p.nangles, 4) * 2 : 0;
     blocks[13] = ceil_div(p.W, 32) * ceil_div(p.H, 32);
     blocks[14] = chunked ? 0 : blocks[13];
-    blocks[12] = marches(p) ? 0 : ceil_div(p.det, 32) * ceil_div(p.nangles, 8);
+    blocks[12] = batch_marches(p) ? 0 : ceil_div(p.det, 32) * ceil_div(p.nangles, 8);
 }
 
 bool batch_chunked(const Plan2d &p) {
