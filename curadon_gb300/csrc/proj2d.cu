@@ -1915,12 +1915,15 @@ static bool bwd_direct(const Plan2d &p) {
 // the 32 views of a staged pass, for as many warps (direct kernel) or CTAs of a
 // cluster to share a tile's views.  The count of groups that gives the SMs the
 // most even load: the fullest SM has ceil(blocks / SMs) blocks of (passes +
-// 0.3 for the start and the end), and fewer than three resident blocks (five
-// of clusters, which do not fill every slot) leave it waiting on latency.
+// 0.3 for the start and the end; a last pass of few views costs one block 0.6 and
+// its views' share), and fewer than three resident blocks (five of clusters, which
+// do not fill every slot) leave it waiting on latency.
 // One group / the rule's, us: 512^2 x 512 116.8 / 68.5, 640^2 x 640 223 / 113,
 // 768^2 x 768 311 / 184, 1024^2 x 1024 490 / 408, 1280^2 x 1280 895 / 771,
 // 2048^2 x 2048 (no quarter turns) 3143 / 2915; 2048^2 x 360 564 and 1024^2 x
-// 90 52.5 keep one (eight: 604, 53.6).  The quarter-turn kernel keeps one: its
+// 90 52.5 keep one (eight: 604, 53.6), as do 33 views (two groups / one): 512^2
+// 14.2 / 11.2, 800^2 25.5 / 17.6, 1000^2 33.7 / 22.6 (56 views 14.2 / 15.7, 25.6 /
+// 25.1, 33.9 / 32.5).  The quarter-turn kernel keeps one: its
 // blocks are already even (2048^2 2672, two groups 2740).
 int bwd_group_views(const Plan2d &p) {
     const int passes = ceil_div(p.nangles, kSmViews);
@@ -1933,7 +1936,9 @@ int bwd_group_views(const Plan2d &p) {
     for (int g = 1; g <= kClusterGroups; ++g) {
         const int per = ceil_div(passes, g);
         const long long blocks = tiles * ceil_div(passes, per);
-        const double time = (double)std::max((blocks + sms - 1) / sms, g == 1 ? 3LL : 5LL) * (per + 0.3);
+        const double work = g == 1 ? std::min<double>(per, p.nangles / (double)kSmViews + 0.6) : per;
+        const double time =
+            (double)std::max((blocks + sms - 1) / sms, g == 1 ? 3LL : 5LL) * (work + 0.3);
         if (g == 1 || time < best_time) best = per, best_time = time;
     }
     return best >= passes ? p.nangles : best * kSmViews;

@@ -51,7 +51,8 @@ def test_split_views_nonfinite(cuda_device, n, views):
     assert torch.equal(torch.nan_to_num(alone), torch.nan_to_num(batched))
 
 
-@pytest.mark.parametrize("n,views", [(64, 360), (120, 700), (300, 400), (640, 640), (900, 450)])
+@pytest.mark.parametrize("n,views", [(64, 360), (120, 700), (300, 400), (640, 640), (900, 450),
+                                     (800, 33), (600, 48)])
 def test_a_large_volume_is_rounded_once(cuda_device, n, views):
     """However many groups a pixel's views are summed in, a value that the volume
     holds already takes one rounding of the result (2^-24 of it) and one of the
