@@ -678,7 +678,10 @@ struct AxViewParams {
 // over 32 (x) x 8 (z) voxels, each warp on a 4 x 8 patch, so that the 8 lanes
 // of a 16-byte load's wavefront (4 x 2 voxels) read a compact piece of the
 // projection (8 x 4 patches: 58.6 ms against 57.9 at 512^3 x 720, 3.91 against
-// 3.87 at 256^3 x 360; 16 x 2: 59.9); blocks are visited in bricks of 2 x 8 x 8
+// 3.87 at 256^3 x 360; 16 x 2: 59.9).  With few views the volume's rows count for
+// more, and a warp takes 8 x 4 (4 x 8 / 8 x 4, us: 256^3 x 1 view 59.8 / 48.0, x 16
+// 205 / 200, x 60 644 / 644; 64 problems of 24^3 x 30 105 / 92): `few`, the same for
+// all the views that one block walks over.  Blocks are visited in bricks of 2 x 8 x 8
 // tiles like k_bwd3d.  The per-view tables are a kernel parameter, read
 // through the constant cache uniformly across the warp: no shared-memory
 // staging or barriers, and the table reads stay off the L1's register
@@ -692,7 +695,7 @@ __device__ __forceinline__ void bwd3d_ax_block(float *__restrict__ vol,
                                                const float4 *__restrict__ SQ, const Tab &tab,
                                                int nv, float num, float su, float sv, int X,
                                                int Y, int Z, int U, int V, int tiles_x,
-                                               int tiles_y, int tiles_z, int lin) {
+                                               int tiles_y, int tiles_z, int lin, bool few) {
     constexpr int BX = 2, BY = 8, BZ = 8;
     const int bricks_x = (tiles_x + BX - 1) / BX, bricks_y = (tiles_y + BY - 1) / BY;
     const int brick = lin / (BX * BY * BZ), in = lin % (BX * BY * BZ);
@@ -703,7 +706,8 @@ __device__ __forceinline__ void bwd3d_ax_block(float *__restrict__ vol,
 
     const int tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5;
-    const int x = tx_ * 32 + warp * 4 + (lane & 3), z = tz_ * 8 + (lane >> 2);
+    const int x = tx_ * 32 + (few ? (warp & 3) * 8 + (lane & 7) : warp * 4 + (lane & 3));
+    const int z = tz_ * 8 + (few ? (warp >> 2) * 4 + (lane >> 3) : lane >> 2);
     const int y0 = ty_ * RUN;
     const float fx = (float)x, fz = (float)z, fy0 = (float)y0;
     const int PU = U + 2 * kP3, PV = V + 2 * kP3;
@@ -760,7 +764,9 @@ __device__ __forceinline__ void bwd3d_ax_block(float *__restrict__ vol,
     }
 }
 
-template <int RUN, int MINB>
+constexpr int kAxFew = 64;  // views below which a warp takes 8 x 4 voxels
+
+template <int RUN, int MINB, bool FEW>
 __global__ void __launch_bounds__(256, MINB)
     k_bwd3d_ax(float *__restrict__ vol, const float4 *__restrict__ SQ,
                 const __grid_constant__ AxViewParams tab, int nv, float num, float su, float sv,
@@ -770,7 +776,7 @@ __global__ void __launch_bounds__(256, MINB)
         p0 = tab.p0[j], p1 = tab.p1[j], p2 = tab.p2[j];
     };
     bwd3d_ax_block<RUN>(vol, SQ, param_tab, nv, num, su, sv, X, Y, Z, U, V, tiles_x, tiles_y,
-                        tiles_z, blockIdx.x);
+                        tiles_z, blockIdx.x, FEW);
 }
 
 }  // namespace
@@ -891,7 +897,7 @@ int launch_backward3d(const Plan3d &p, float *vol, const float *sino, cudaStream
         const int bricks = ceil_div(tiles_x, 2) * ceil_div(tiles_y, 8) * ceil_div(tiles_z, 8);
         const size_t plane = (size_t)(p.U + 2 * kP3) * (p.V + 2 * kP3);
         // runs of 8 voxels at <= 48 registers (5 blocks per SM)
-        auto kernel = k_bwd3d_ax<run, 5>;
+        auto kernel = p.nangles < kAxFew ? k_bwd3d_ax<run, 5, true> : k_bwd3d_ax<run, 5, false>;
         // the view tables travel as a kernel parameter, kAxViews per launch
         AxViewParams tab{};
         for (int c0 = 0; c0 < p.nangles; c0 += kAxViews) {
@@ -1002,7 +1008,8 @@ __global__ void __launch_bounds__(256, 5)
             p0 = __ldg(a0 + j), p1 = __ldg(a1 + j), p2 = __ldg(a2 + j);
         };
         bwd3d_ax_block<RUN>(q.vol, q.sinoQ + plane * c0, tab, nv, q.num, q.su, q.sv, q.X, q.Y,
-                            q.Z, q.U, q.V, q.tiles_x, q.tiles_y, q.tiles_z, lin);
+                            q.Z, q.U, q.V, q.tiles_x, q.tiles_y, q.tiles_z, lin,
+                            q.P < kAxFew);
     }
 }
 

@@ -29,3 +29,21 @@ def test_axial_equals_general(cuda_device, monkeypatch, n, views, det):
         out.append(v.double())
     assert out[1].abs().max() > 0
     assert (out[0] - out[1]).abs().max() <= views * 2.0 ** -18 * (max(det) + n)
+
+
+@pytest.mark.parametrize("views", [63, 64])  # a warp's 8 x 4 and 4 x 8 voxels
+@pytest.mark.parametrize("shape", [(1, 1, 1), (9, 3, 31), (7, 9, 33), (17, 8, 70)])
+def test_axial_patches_cover_the_volume(cuda_device, monkeypatch, shape, views):
+    n, det = max(shape), (19, 45)
+    g = cone_config(n, views, 1)
+    g.update(vol_shape=shape, det_shape=det)
+    y = torch.rand((views, *det), device=cuda_device,
+                   generator=torch.Generator(cuda_device).manual_seed(n))
+    out = []
+    for algo in ("ax8m5", "pair"):
+        monkeypatch.setenv("CURADON_GB300_ALGO", "bwd3d=" + algo)
+        v = torch.zeros(shape, device=cuda_device)
+        backward(y, v, ConeGeometry(**g))
+        out.append(v.double())
+    assert out[1].abs().max() > 0
+    assert (out[0] - out[1]).abs().max() <= views * 2.0 ** -18 * (max(det) + n)
