@@ -168,6 +168,8 @@ int cg_batch2d_create(cg_batch2d **batch, cg_plan2d *const *plans, float *const 
     std::vector<Prob2d> probs(count);
     std::vector<int> starts(kBatchStages * (count + 1), 0);
     long long totals[kBatchStages] = {};
+    double march_shares = 0.0;
+    for (int i = 0; i < count; ++i) march_shares += march_share(*plans[i]);
     for (int i = 0; i < count; ++i) {
         const Plan2d &p = *plans[i];
         Prob2d &q = probs[i];
@@ -183,7 +185,7 @@ int cg_batch2d_create(cg_batch2d **batch, cg_plan2d *const *plans, float *const 
         q.bwd_sym = p.bwd_sym;
         q.bwd_per = bwd_group_views(p);
         int blocks[kBatchStages];
-        batch_blocks(p, blocks);
+        batch_blocks(p, march_shares, blocks);
         for (int st = 0; st < kBatchStages; ++st) {
             starts[st * (count + 1) + i] = (int)totals[st];
             totals[st] += blocks[st];

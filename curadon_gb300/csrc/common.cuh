@@ -323,8 +323,9 @@ struct SideStream {
 int launch_relayout_sino2d(const Plan2d &p, const void *sino, bool half, cudaStream_t s);
 // batches (proj2d.cu): blocks of each stage of one problem, and the launch of
 // one direction over a batch whose starts hold kBatchStages x (count + 1) block
-// starts
-void batch_blocks(const Plan2d &p, int blocks[kBatchStages]);
+// starts (march_shares: the sum of the problems' march_share)
+void batch_blocks(const Plan2d &p, double march_shares, int blocks[kBatchStages]);
+double march_share(const Plan2d &p);
 // true where the batched "plans" forward runs the plan's chunked shape
 bool batch_chunked(const Plan2d &p);
 int launch_batch2d(const Prob2d *probs, const int *starts, const int totals[kBatchStages],

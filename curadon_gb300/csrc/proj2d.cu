@@ -777,23 +777,31 @@ __global__ void __launch_bounds__(128, 5)
                  blockIdx.y, blockIdx.z);
 }
 
-// Its window table packs columns in 16 bits, its grid 4 views per row.  Rays of
-// less than 256 samples do not pay for a bundle's set-up once there are more
-// bundles than nine for every SM, nor do the shortest at all.  Ray by ray / this,
-// us: 32^2 x 8 views 10.2 / 14.5, 64^2 x 90 25.1 / 18.6, x 720 (720 bundles) 23.6 /
-// 24.0, x 1440 24.2 / 37.1, 128^2 x 720 (1080) 41.6 / 37.6, x 1440 (2160) 53.4 /
-// 66.4, 200^2 x 360 (900) 66.7 / 45.6, x 720 (1800) 60.2 / 67.8, 256^2 x 720 (2160)
-// 95 / 88, x 1440 149 / 141.
-static bool marches(const Plan2d &p) {
-    const long long bundles = 2LL * ceil_div(p.det, 64) * ceil_div(p.nangles, 4);
-    const int side = std::max(p.W, p.H);
+// Its window table packs columns in 16 bits, its grid 4 views per row.
+static bool can_march(const Plan2d &p) {
     return p.fwd_march && std::max(p.pitchA(), p.pitchB()) < 32768 &&
-           ceil_div(p.nangles, 4) <= 65535 &&
-           (side >= 256 || (side >= 64 && bundles <= 9LL * sm_count()));
+           ceil_div(p.nangles, 4) <= 65535;
 }
-// In a batch, small images have company: their bundles are many (64 of 64^2 x 30
-// views 45 us ray by ray, 63 so; 16 of 96^2 x 90 51, 62).
-static bool batch_marches(const Plan2d &p) { return marches(p) && std::max(p.W, p.H) >= 256; }
+
+// A bundle of short rays does not pay for its set-up once there are bundles
+// enough to fill the SMs: a plan's share of them, for images of 64 to 255 pixels
+// (larger ones always march, smaller ones never).  They march while the shares
+// of a launch come to one.  Ray by ray / this, us: 32^2 x 8 views 10.2 / 14.5;
+// 64^2 x 90 (share 0.1) 25.1 / 18.6, x 720 (1.0) 23.6 / 24.0, x 1440 (2.1) 24.2 /
+// 37.1; 128^2 x 720 (0.8) 41.6 / 37.6, x 1440 (1.6) 53.4 / 66.4; 200^2 x 360 (0.7)
+// 66.7 / 45.6, x 720 (1.3) 60.2 / 67.8; 256^2 x 720 95 / 88, x 1440 149 / 141; in
+// batches, 2 of 128^2 x 128 (0.3) 45 / 31, 64 of 64^2 x 30 (2.9) 45 / 63, 16 of
+// 96^2 x 90 (2.1) 51 / 62.
+double march_share(const Plan2d &p) {
+    const int side = std::max(p.W, p.H);
+    if (side < 64 || side >= 256 || !can_march(p)) return 0.0;
+    const double bundles = 2.0 * ceil_div(p.det, 64) * ceil_div(p.nangles, 4);
+    return bundles / (std::min(9.0, side / 14.0) * sm_count());
+}
+static bool marches(const Plan2d &p, double share) {
+    return can_march(p) && (std::max(p.W, p.H) >= 256 ||
+                            (std::max(p.W, p.H) >= 64 && share <= 1.0));
+}
 
 static size_t cslab_smem(int stride) { return 2 * sizeof(float2) * (kCsRows + 1) * stride; }
 
@@ -1731,7 +1739,7 @@ __global__ void __launch_bounds__(256, 4)
 
 // Blocks of each batched stage for one problem (the launch shapes of the
 // single-problem kernels above).
-void batch_blocks(const Plan2d &p, int blocks[kBatchStages]) {
+void batch_blocks(const Plan2d &p, double march_shares, int blocks[kBatchStages]) {
     blocks[0] = ceil_div(p.W + 2 * kPad, kTile) * ceil_div(p.H + 2 * kPad, kTile);
     blocks[1] = tex_blocks(p);
     blocks[2] = (int)ceil_div((long long)p.pitchS() * p.nangles, 256);
@@ -1750,10 +1758,11 @@ void batch_blocks(const Plan2d &p, int blocks[kBatchStages]) {
     blocks[7] = chunked ? blocks[0] : 0;
     blocks[8] = chunked ? ceil_div(p.det, 128) * ceil_div(p.nangles, 8) * 2 : 0;
     blocks[9] = chunked ? 0 : blocks[1];
-    blocks[11] = batch_marches(p) ? ceil_div(p.det, 64) * ceil_div(p.nangles, 4) * 2 : 0;
+    const bool march = marches(p, march_shares);
+    blocks[11] = march ? ceil_div(p.det, 64) * ceil_div(p.nangles, 4) * 2 : 0;
     blocks[13] = ceil_div(p.W, 32) * ceil_div(p.H, 32);
     blocks[14] = chunked ? 0 : blocks[13];
-    blocks[12] = batch_marches(p) ? 0 : ceil_div(p.det, 32) * ceil_div(p.nangles, 8);
+    blocks[12] = march ? 0 : ceil_div(p.det, 32) * ceil_div(p.nangles, 8);
 }
 
 bool batch_chunked(const Plan2d &p) {
@@ -1848,7 +1857,7 @@ int launch_relayout2d(const Plan2d &p, const void *vol, bool half, cudaStream_t 
 }
 
 int launch_forward2d(const Plan2d &p, float *sino, cudaStream_t s) {
-    if (marches(p)) {
+    if (marches(p, march_share(p))) {
         const size_t smem = cslab_smem(kCsSmallCols);
         if (int rc = ensure_smem_attr((const void *)k_fwd2d_march, (int)smem)) return rc;
         const dim3 grid(ceil_div(p.det, 64), ceil_div(p.nangles, 4), 2);

@@ -80,3 +80,15 @@ def test_forward_block_shapes_the_ray_by_ray_kernel(cuda_device, monkeypatch):
         out = torch.full_like(expect, -1.0)
         forward_2d(vol, out, plan)
         assert torch.equal(out, expect)
+
+
+@pytest.mark.parametrize("count", [2, 40])  # in bundles; too many of them: ray by ray
+def test_small_problems_of_a_batch(cuda_device, count):
+    geoms = [FanGeometry(**fan_config(72 + k % 3, 120)) for k in range(count)]
+    gen = torch.Generator(device=cuda_device).manual_seed(count)
+    vols = [torch.rand(tuple(int(v) for v in g.vol_shape), device=cuda_device, generator=gen)
+            for g in geoms]
+    sinos = [torch.full(g.sinogram_shape(), -1.0, device=cuda_device) for g in geoms]
+    Batch2d(geoms, vols, sinos, forward="registers").forward()
+    for g, v, s in zip(geoms, vols, sinos):
+        assert torch.equal(s, forward(v, torch.full_like(s, -2.0), g, exact=True))
